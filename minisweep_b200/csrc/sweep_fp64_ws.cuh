@@ -76,6 +76,7 @@ struct Fp64Params {
   const int* tasks;
   long long ntask;
   SyncArgs sy;
+  int rw;  // row kernel: rows per pipeline (8, 4 or 2)
 };
 
 // Many problems per launch.  Tasks of all problems share one table with

@@ -18,6 +18,7 @@
 
 #include "internal.h"
 #include "sweep_fp64_chain.cuh"
+#include "sweep_fp64_row.cuh"
 #include "sweep_fp64_ws.cuh"
 #include "sweep_mixed_tc.cuh"
 
@@ -38,7 +39,12 @@ struct Variant {
   size_t entry_bytes = 0;  // one face entry (octant, group pair, position)
   int tx = 0, ty = 0, nch = 0, threads = 0;
   int pass = 64;  // angles swept per launch (na above it is swept in passes)
-  int kernel = 0; // FP64: 0 staged, 1 chained wavefront
+  int kernel = 0;  // FP64: 0 staged, 1 chained wavefront, 2 rows
+  // row kernel: the bodies for passes of 8, 16, 24, 32 angles, rows per pipeline
+  KernelFn row_fn[4] = {nullptr, nullptr, nullptr, nullptr};
+  size_t row_smem[4] = {0, 0, 0, 0};
+  int rw = 0;
+  int gpt() const { return rw ? 8 / rw : 1; }  // group pairs per task
   bool valid() const { return fn || mix; }
   const void* func() const { return fn ? (const void*)fn : (const void*)mix; }
 };
@@ -81,6 +87,43 @@ Variant make_chain_variant() {
   v.pass = 32;
   v.kernel = 1;
   return v;
+}
+
+// The row kernel (sweep_fp64_row.cuh): rw rows of 4 cells per pipeline,
+// 8 / rw pipelines (group pairs) per CTA.
+template <int NM_>
+Variant make_row_variant(int rw, int na) {
+  Variant v;
+  v.row_fn[0] = sweep_fp64_row_kernel<NM_, 1>;
+  v.row_fn[1] = sweep_fp64_row_kernel<NM_, 2>;
+  v.row_fn[2] = sweep_fp64_row_kernel<NM_, 3>;
+  v.row_fn[3] = sweep_fp64_row_kernel<NM_, 4>;
+  v.row_smem[0] = RowCfg<NM_, 1>::smem_bytes();
+  v.row_smem[1] = RowCfg<NM_, 2>::smem_bytes();
+  v.row_smem[2] = RowCfg<NM_, 3>::smem_bytes();
+  v.row_smem[3] = RowCfg<NM_, 4>::smem_bytes();
+  static_assert(RowCfg<NM_, 4>::smem_bytes() <= 227 * 1024, "shared memory budget");
+  const int nt = std::min(4, (na + 7) / 8);  // of the widest pass
+  v.fn = v.row_fn[nt - 1];
+  v.smem = v.row_smem[nt - 1];
+  v.entry_bytes = (size_t)nt * 64 * sizeof(double);
+  v.tx = 4;
+  v.ty = rw;
+  v.nch = 1;
+  v.threads = RowCfg<NM_, 4>::NTH;
+  v.pass = 32;
+  v.kernel = 2;
+  v.rw = rw;
+  return v;
+}
+
+Variant pick_row(int nm, int na, int rw) {
+  switch (nm) {
+    case 4: return make_row_variant<4>(rw, na);
+    case 8: return make_row_variant<8>(rw, na);
+    case 16: return make_row_variant<16>(rw, na);
+    default: return Variant();
+  }
 }
 
 // FP64 tile shapes: 4 x 2 (tile 42, the default) or 2 x 4 (tile 24) cell
@@ -277,6 +320,23 @@ struct SweeperImpl {
 // ranges whose contributions add up in vo.
 static int pass_angles(const SweeperImpl& S) { return S.var.pass; }
 
+// Rows per pipeline of the row kernel.  8 rows in one pipeline move the fewest
+// y faces and leave the most CTAs to a phase; where a region's rows leave many
+// of the 8 warps idle and there are tasks enough for every CTA all the same
+// (4 rounds or more), shorter pipelines share the CTA between group pairs.
+// Measured, ms per sweep with 8, 4, 2 rows:
+//   64 x 64 x 64, ne 64   57.3  60    63.0     48 x 20 x 48, ne 32   7.29  6.43  6.45
+//   24 x 24 x 24, ne 8    0.78  0.85  0.97     40 x 6 x 40, ne 64    4.30  2.99  3.13
+//   10 x 10 x 10, ne 30   0.31  0.36  0.36     20 x 4 x 6, ne 64     0.42  0.35  0.33
+static int pick_rows(const Dimensions& d, int ngp, int nsm) {
+  const int hx = (d.ncell_x + 1) / 2, h0 = (d.ncell_y + 1) / 2, h1 = d.ncell_y / 2;
+  auto up = [](int n, int m) { return (n + m - 1) / m; };
+  if (8LL * up(hx, 4) * up(h0, 8) * ngp < 4LL * nsm) return 8;
+  auto cost = [&](int rw, double faces) { return (up(h0, rw) + up(h1, rw)) * rw * faces; };
+  const double c8 = cost(8, 1.15), c4 = cost(4, 1.05), c2 = cost(2, 1.45);
+  return c8 <= c4 && c8 <= c2 ? 8 : c4 <= c2 ? 4 : 2;
+}
+
 // Schedule, device task table and grid of one compiled tile shape, with a
 // window of `window` x SMs consecutive tasks between a tile and its downwind
 // neighbour in the table.
@@ -284,8 +344,9 @@ static int setup_plan(const SweeperImpl& S, const Variant& var, int window, Sche
                       int*& d_tasks, int& grid) {
   const Dimensions& dims = S.dims;
   int rc, occ = 0;
-  gp_block = pick_gp_block(dims.ncell_x, dims.ncell_y, S.ngp, var.tx, var.ty, window * S.nsm);
-  if ((rc = build_schedule(dims.ncell_x, dims.ncell_y, dims.ncell_z, S.ngp, var.tx, var.ty, gp_block, sched)))
+  const int nblk = (S.ngp + var.gpt() - 1) / var.gpt();  // blocks of group pairs, one per task
+  gp_block = pick_gp_block(dims.ncell_x, dims.ncell_y, nblk, var.tx, var.ty, window * S.nsm);
+  if ((rc = build_schedule(dims.ncell_x, dims.ncell_y, dims.ncell_z, nblk, var.tx, var.ty, gp_block, sched)))
     return rc;
   const long long ntask = sched.ntask();
   if (ntask >= (1LL << 31) - SY_PROGRESS) return set_error(MSB_ERR_ARG, "too many tasks");
@@ -296,6 +357,14 @@ static int setup_plan(const SweeperImpl& S, const Variant& var, int window, Sche
   if ((rc = cuda_check(cudaFuncSetAttribute(var.func(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)var.smem),
                        "cudaFuncSetAttribute")))
     return rc;
+  const int rem = dims.na % 32;  // the row kernel's body for a last pass of fewer angles
+  if (var.rw && rem) {
+    const int b = (rem + 7) / 8 - 1;
+    if ((rc = cuda_check(cudaFuncSetAttribute((const void*)var.row_fn[b], cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                              (int)var.row_smem[b]),
+                         "cudaFuncSetAttribute")))
+      return rc;
+  }
   if ((rc = cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, var.func(), var.threads, var.smem),
                        "occupancy")))
     return rc;
@@ -323,13 +392,30 @@ static int impl_create(SweeperImpl& S, const Dimensions& dims, int precision, in
   if ((rc = cuda_check(cudaGetDevice(&dev), "cudaGetDevice"))) return rc;
   if ((rc = cuda_check(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev), "SM count"))) return rc;
   S.nsm = nsm;
+  // no flag asks for a shape or a kernel: the row kernel
+  if (precision == 0 && kernel == 0 && tile == 0 && angle_pass == 0 && !autotune)
+    S.var = pick_row(dims.nm, dims.na, pick_rows(dims, S.ngp, nsm));
   if ((rc = setup_plan(S, S.var, S.window, S.sched, S.gp_block, S.d_tasks, S.grid))) return rc;
   long long ntask = S.sched.ntask();
   if (autotune) {
-    // candidates: both FP64 kernels (the staged one with 32- and 64-angle
-    // passes when na > 32) x both tile shapes x task windows of 4, 8 and 16
-    // x SMs, besides the sweeper's own plan
+    // candidates: the staged and the chained kernel (the staged one with 32-
+    // and 64-angle passes when na > 32) x both tile shapes x task windows of
+    // 4, 8 and 16 x SMs, besides the sweeper's own plan; and the row kernel,
+    // with pipelines of more than 2 rows where a region has more than 4
     S.autotune = true;
+    for (int rw : {8, 4, 2}) {
+      if (rw > 2 && (dims.ncell_y + 1) / 2 <= 4) continue;
+      AltPlan a;
+      a.var = pick_row(dims.nm, dims.na, rw);
+      a.window = S.window;
+      a.l2_hints = S.l2_hints;
+      if ((rc = setup_plan(S, a.var, a.window, a.sched, a.gp_block, a.d_tasks, a.grid))) {
+        cudaFree(a.d_tasks);
+        return rc;
+      }
+      ntask = std::max(ntask, a.sched.ntask());
+      S.alts.push_back(std::move(a));
+    }
     const int windows[3] = {4, 8, 16};
     for (int k = 0; k < 3; ++k)
       for (int t = 0; t < 2; ++t)
@@ -453,16 +539,28 @@ static int launch_fp64(SweeperImpl& S, const Variant& var, const int* d_tasks, l
     fill_params<double>(S, P.pr, P, vi_d, d_tasks, ntask);
     P.pr.vo = vo_d;
     P.pr.vo_add = c > 0 ? 1 : 0;  // later passes add to vo in every phase
+    const int a0 = pa * c, nac = std::min(pa, na - a0);
     if (npass > 1) {
-      const int a0 = pa * c, nac = std::min(pa, na - a0);
-      if ((rc = copy_pass_matrices(S, a0, nac, stream))) return rc;
       if (c > 0 && (rc = reset_pass(S, stream))) return rc;
-      P.pr.afm = S.d_afm_c;
-      P.pr.mfa = S.d_mfa_c;
       P.pr.na = nac;
       P.pr.ia_base = a0;
+      if (var.rw) {  // the pass's angles read in place
+        P.pr.afm = S.d_afm + a0;
+        P.pr.mfa = S.d_mfa + (size_t)a0 * S.dims.nm;
+        P.pr.a_stride = na;
+      } else {
+        if ((rc = copy_pass_matrices(S, a0, nac, stream))) return rc;
+        P.pr.afm = S.d_afm_c;
+        P.pr.mfa = S.d_mfa_c;
+      }
     }
-    var.fn<<<grid, var.threads, var.smem, stream>>>(P);
+    if (var.rw) {
+      const int b = (nac + 7) / 8 - 1;
+      P.rw = var.rw;
+      var.row_fn[b]<<<grid, var.threads, var.row_smem[b], stream>>>(P);
+    } else {
+      var.fn<<<grid, var.threads, var.smem, stream>>>(P);
+    }
     if ((rc = cuda_check(cudaGetLastError(), "sweep kernel launch"))) return rc;
   }
   return MSB_OK;
@@ -651,9 +749,11 @@ static int build_slices(SweeperImpl& S, int nslice) {
   const long long n = S.sched.ntask();
   const int* rec = S.sched.rec.data();
   std::vector<long long> index(n, -1);  // task -> its index in its slice
-  for (int k = 0; k <= nslice; ++k) T->gp0.push_back((int)((long long)S.ngp * k / nslice));
+  // a task covers gpt group pairs, which stay in one slice
+  const int gpt = S.var.gpt(), nblk = (S.ngp + gpt - 1) / gpt;
+  for (int k = 0; k <= nslice; ++k) T->gp0.push_back(std::min(S.ngp, (int)((long long)nblk * k / nslice) * gpt));
   for (int k = 0; k < nslice; ++k) {
-    const int g0 = T->gp0[k], g1 = T->gp0[k + 1];
+    const int g0 = T->gp0[k] / gpt, g1 = (T->gp0[k + 1] + gpt - 1) / gpt;
     std::vector<int> out;
     long long m = 0;
     for (long long t = 0; t < n; ++t) {
@@ -1151,7 +1251,8 @@ extern "C" int Sweeper_create_status(Sweeper* sweeper, Dimensions dims, const Qu
   // 1: the first sweep times both FP64 tile shapes and keeps the faster
   const int autotune = Arguments_consume_int_or_default(args, "--autotune", 0);
   if (autotune != 0 && autotune != 1) return msb::set_error(MSB_ERR_ARG, "--autotune must be 0 or 1");
-  // FP64 sweep kernel: 0 = the staged kernel (default), 1 = the chained wavefront
+  // FP64 sweep kernel: 0 = the row kernel, or the staged one where --tile,
+  // --angle_pass or --autotune ask for its shapes; 1 = the chained wavefront
   const int fp64_kernel = Arguments_consume_int_or_default(args, "--fp64_kernel", 0);
   if (fp64_kernel != 0 && fp64_kernel != 1) return msb::set_error(MSB_ERR_ARG, "--fp64_kernel must be 0 or 1");
   // angles per pass of the staged FP64 kernel: 0 or 32 = 32, 64 = two chunks per pass

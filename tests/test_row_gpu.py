@@ -1,0 +1,46 @@
+"""The row FP64 kernel (the default sweep) where its tiles, pipelines and
+angle tiles end: against the staged kernel (`--tile 42`), which sums in the
+same order, bit for bit on random inputs, and against the oracle.  The oracle
+adds a cell's 16 moments and 32 angles in another order: 1e-12 relative, as
+for every FP64 kernel of the library."""
+import numpy as np
+import pytest
+
+import oracle
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+import minisweep_b200 as msb  # noqa: E402
+
+
+def sweep(dims, extra, a, m, vi):
+    nx, ny, nz, ne, na, nm = dims
+    with msb.Problem(f"--ncell_x {nx} --ncell_y {ny} --ncell_z {nz} --ne {ne} --na {na} {extra}", nm=nm) as pb:
+        pb.set_matrices(a, m)
+        return pb.sweep_host(vi), pb.tile()
+
+
+@pytest.mark.parametrize("nx,ny,nz,ne,na,nm,ty", [
+    (1, 1, 1, 1, 1, 16, 8),      # one cell, one group of a pair, one angle
+    (2, 2, 2, 2, 8, 4, 8),       # row width 1, one angle tile
+    (5, 3, 3, 3, 9, 8, 8),       # row widths 3 and 2, two angle tiles
+    (8, 16, 2, 4, 24, 16, 8),    # whole tiles, three angle tiles
+    (9, 17, 5, 5, 32, 16, 8),    # remainders of 1 in both directions
+    (17, 30, 4, 3, 33, 4, 8),    # a second pass of one angle
+    (6, 33, 3, 2, 61, 8, 8),     # a second pass of 29 angles
+    (20, 5, 6, 63, 32, 16, 4),   # 2 pipelines of 4 rows, an odd group count
+    (20, 7, 3, 50, 40, 4, 4),    # ... the last task with one pipeline
+    (20, 4, 6, 64, 32, 16, 2),   # 4 pipelines of 2 rows
+    (33, 3, 2, 61, 17, 8, 2),    # ... rows of 2 and 1, the last task with 3 pipelines
+])
+def test_row_kernel_edges(nx, ny, nz, ne, na, nm, ty):
+    dims = (nx, ny, nz, ne, na, nm)
+    a, m, vi = oracle.random_problem(nx, ny, nz, ne, nm, na, seed=77)
+    vo, tile = sweep(dims, "", a, m, vi)
+    assert (tile["fp64_kernel"], tile["tx"], tile["ty"]) == (2, 4, ty)
+    staged, t0 = sweep(dims, "--tile 42", a, m, vi)
+    assert t0["fp64_kernel"] == 0
+    assert np.array_equal(vo, staged)
+    ref = oracle.sweep(nx, ny, nz, ne, nm, na, a, m, vi)
+    assert np.max(np.abs(vo - ref)) <= 1e-12 * np.max(np.abs(ref))
