@@ -425,9 +425,10 @@ int msb_sweep_noalloc(double* vo_d, const double* vi_d, const double* a_from_m_d
  * are scratch from one device arena of scratch_bytes (0: what all problems
  * need at once, capped at 80 % of the free device memory); problems that do
  * not fit at once reuse the bytes of problems that completed earlier in the
- * same launch.  autotune != 0 times the two tile shapes (4 x 2 and 2 x 4
- * cells) on the median problem of each nm group at creation;
- * those trial sweeps write that problem's vo.  Asynchronous calls run on the
+ * same launch.  Every problem is swept by the row kernel in pipelines of 8, 4
+ * or 2 rows of 4 cells (class_tx x class_ty of the info is the smallest, 4 x 2);
+ * autotune != 0 times these on the median problem of each nm group at
+ * creation; those trial sweeps write that problem's vo.  Asynchronous calls run on the
  * given stream (a cudaStream_t, NULL = the legacy default stream); their
  * device status is checked by msb_batch_sync. */
 typedef struct {

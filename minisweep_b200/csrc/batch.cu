@@ -6,27 +6,29 @@
 // them in ONE launch of a persistent kernel:
 //
 //   * Every problem gets the task schedule a Sweeper would build for it
-//     (schedule.cpp).  Problems are grouped in classes, one per compiled
-//     kernel body (moment count, 32-angle chunks, tile shape); the kernel's
-//     CTAs work through the classes in kind order, each class a contiguous
-//     range of one task table with global task ids.
+//     (schedule.cpp), cut for the row kernel's pipelines.  Problems are
+//     grouped in classes, one per compiled kernel body (moment count, angle
+//     tiles of the first pass); the kernel's CTAs work through the classes in
+//     kind order, each class a contiguous range of one task table with global
+//     task ids.
 //   * The face planes are scratch that a problem needs only while it runs.
 //     They come from one arena, placed first-fit in admission order; a problem
 //     placed over bytes that earlier problems used waits, on the device, until
 //     those problems have completed every task (a per-problem counter).
 //   * The order of the table comes from a host-side list-scheduling
-//     simulation: one worker per SM, task durations proportional to their
-//     wavefront steps, a same-phase neighbour tile released one tile
-//     diagonal after its upwind tile starts (the kernel pipelines them plane
-//     by plane), other dependencies released at completion, problems admitted
+//     simulation: one worker per SM, task durations proportional to the
+//     cells of a row, a same-phase neighbour tile released once the first
+//     plane is through every row (the kernel pipelines them plane by plane),
+//     other dependencies released at completion, problems admitted
 //     while the arena has room.  Tasks enter the table in simulated start
 //     order, so dependencies always precede their dependents and the CTAs,
 //     which grab tasks in table order, rarely wait.
 //   * The reference driver's iteration loop (runner.c:148-155: niterations
 //     sweeps, swapping vi and vo) runs as a CUDA graph of one launch per
 //     iteration, captured once per iteration count.
-//   * The tile shape of each class is chosen by timing both shapes on the
-//     class's median problem (autotune), or defaults to 4 x 2.
+//   * Every problem's rows per pipeline come from a rule (pick_rows), or
+//     (autotune) each moment count's from timing the rule's and the fixed
+//     choices on its median problem.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -41,12 +43,81 @@
 #include <vector>
 
 #include "internal.h"
-#include "sweep_fp64_ws.cuh"
+#include "sweep_fp64_row.cuh"
 
 namespace msb {
+
+// Batched sweep: one class per moment count and angle tiles of a problem's
+// first (widest) pass; every task takes its problem's pipeline shape.  The
+// CTAs work through the classes in kind order; a CTA moves on when its
+// class's table is exhausted, so a task only ever waits on tasks that CTAs
+// hold and advance.
+constexpr int batch_kind(int nm, int nt) { return (nm == 4 ? 0 : nm == 8 ? 4 : 8) + 4 - nt; }
+
+// F(NM, NT) in increasing kind order.
+#define MSB_ROW_BATCH_KINDS(F) \
+  F(4, 4) F(4, 3) F(4, 2) F(4, 1) F(8, 4) F(8, 3) F(8, 2) F(8, 1) F(16, 4) F(16, 3) F(16, 2) F(16, 1)
+
+// Between two classes: every warp of the CTA is done with the previous
+// class's shared memory (a barrier that warps reach from their own role's
+// code, so the non-aligned form), thread 0 swaps the barrier sets, and nobody
+// starts the new class before that.
+__device__ __forceinline__ void row_batch_switch(const Fp64Batch& P, int c, double* smem) {
+  asm volatile("barrier.sync 0;" ::: "memory");
+  if (threadIdx.x == 0) {
+    for (int k = 0; k < 2; ++k) {
+      const bool init = k == 1;
+      const int cc = init ? c : c - 1;
+      if (cc < 0 || cc >= P.nclass) continue;
+      switch (P.cls_kind[cc]) {
+#define MSB_K(NM, NT) \
+  case batch_kind(NM, NT): row_setup<NM, NT>(smem, init); break;
+        MSB_ROW_BATCH_KINDS(MSB_K)
+#undef MSB_K
+        default: break;
+      }
+    }
+  }
+  asm volatile("barrier.sync 0;" ::: "memory");
+}
+
+// The classes of a launch come in increasing kind order (the host sorts them
+// so), and the kernel visits the kinds in that order, one straight-line
+// region per kind.
+__global__ void __launch_bounds__(384, 1) sweep_fp64_row_batch_kernel(const Fp64Batch P) {
+  extern __shared__ __align__(128) double smem[];
+  if (blockIdx.x == 0 && threadIdx.x == 0) P.ptime[P.nprob] = global_ns();
+  int c = 0;
+  if ((threadIdx.x >> 5) >= 8) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(80));
+#define MSB_K(NM, NT)                                              \
+  if (c < P.nclass && P.cls_kind[c] == batch_kind(NM, NT)) {       \
+    row_batch_switch(P, c, smem);                                  \
+    row_producers<NM, NT, true>(P, c, smem);                       \
+    ++c;                                                           \
+  }
+    MSB_ROW_BATCH_KINDS(MSB_K)
+#undef MSB_K
+  } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(208));
+#define MSB_K(NM, NT)                                              \
+  if (c < P.nclass && P.cls_kind[c] == batch_kind(NM, NT)) {       \
+    row_batch_switch(P, c, smem);                                  \
+    row_compute<NM, NT, true>(P, smem);                                  \
+    ++c;                                                           \
+  }
+    MSB_ROW_BATCH_KINDS(MSB_K)
+#undef MSB_K
+  }
+}
+
+// Dynamic shared memory of the batched kernel: the largest body.
+constexpr size_t row_batch_smem() { return RowCfg<16, 4>::smem_bytes(); }
+static_assert(RowCfg<8, 4>::smem_bytes() <= row_batch_smem() && RowCfg<4, 4>::smem_bytes() <= row_batch_smem(),
+              "largest body");
+
 namespace {
 
-constexpr int kBatchStages = 4;
 constexpr long long kBatchTimeoutNs = 4000000000LL;
 constexpr size_t kAlign = 256;
 
@@ -63,6 +134,8 @@ struct ProbPlan {
   int user = 0, pass = 0, npass = 1, a0 = 0, nac = 0;
   int prev = -1, next = -1;  // entries of the neighbouring passes
   int nch = 0, ngp = 0, kind = 0, cls = 0, tx = 4, ty = 2;
+  int rw = 0;  // rows per pipeline of the row kernel; 0: planned for the given tile only (no device)
+  int nt = 4;  // angle tiles of the class: those of the problem's first pass
   Schedule sched;
   size_t face_bytes[3] = {0, 0, 0};
   size_t scratch = 0;      // bytes of the three face arrays
@@ -80,6 +153,21 @@ struct ClassInfo {
 
 // relative cost of one wavefront step of a task (one cell column per warp)
 double step_cost(int nm, int nch) { return (0.3 + 0.7 * nm / 16.0) * nch; }
+
+// Duration of a task and the delay until its first plane is through every
+// row.  Row kernel: in cells of a warp, the rows one cell apart.
+void task_times(const ProbPlan& P, const int* r, double* dur, double* plane_delay) {
+  const int w = r[TK_X1] - r[TK_X0], h = r[TK_Y1] - r[TK_Y0], nz = r[TK_Z1] - r[TK_Z0];
+  if (P.rw) {
+    const double c = step_cost(P.d.nm, 1) * (0.2 + 0.2 * P.nt) / 4.0;
+    *dur = c * (nz * w + h - 1);
+    *plane_delay = c * (w + h - 1);
+  } else {
+    const double c = step_cost(P.d.nm, P.nch);
+    *dur = c * (nz + w + h - 2);
+    *plane_delay = c * (w + h - 1);
+  }
+}
 
 }  // namespace
 
@@ -157,22 +245,23 @@ int plan_problem(ProbPlan& P, int nsm) {
   const msb_problem& d = P.d;
   P.nch = 1;
   P.ngp = (d.ne + 1) / 2;
+  const int gpt = P.rw ? 8 / P.rw : 1, nblk = (P.ngp + gpt - 1) / gpt;  // group pairs per task, tasks across groups
   // the same task window as a single problem's schedule (4 x SMs)
-  const int gpb = pick_gp_block(d.ncell_x, d.ncell_y, P.ngp, P.tx, P.ty, 4 * nsm);
-  int rc = build_schedule(d.ncell_x, d.ncell_y, d.ncell_z, P.ngp, P.tx, P.ty, gpb, P.sched);
+  const int gpb = pick_gp_block(d.ncell_x, d.ncell_y, nblk, P.tx, P.ty, 4 * nsm);
+  int rc = build_schedule(d.ncell_x, d.ncell_y, d.ncell_z, nblk, P.tx, P.ty, gpb, P.sched);
   if (rc) return rc;
-  const size_t per = (size_t)NOCTANT * P.ngp * (size_t)P.nch * 256 * sizeof(double);
+  const size_t per = (size_t)NOCTANT * P.ngp * (size_t)P.nt * 64 * sizeof(double);
   P.face_bytes[0] = align_up(per * d.ncell_y * d.ncell_x);
   P.face_bytes[1] = align_up(per * d.ncell_z * d.ncell_x);
   P.face_bytes[2] = align_up(per * d.ncell_z * d.ncell_y);
   P.scratch = P.face_bytes[0] + P.face_bytes[1] + P.face_bytes[2];
-  double steps = 0.0;
+  P.work = 0.0;
   const long long n = P.sched.ntask();
   for (long long t = 0; t < n; ++t) {
-    const int* r = &P.sched.rec[t * MSB_TASK_INTS];
-    steps += (r[TK_Z1] - r[TK_Z0]) + (r[TK_X1] - r[TK_X0]) + (r[TK_Y1] - r[TK_Y0]) - 2;
+    double dur, pd;
+    task_times(P, &P.sched.rec[t * MSB_TASK_INTS], &dur, &pd);
+    P.work += dur;
   }
-  P.work = steps * step_cost(d.nm, P.nch);
   return MSB_OK;
 }
 
@@ -273,14 +362,14 @@ int simulate_and_order(BatchImpl& B) {
   std::vector<int> dcount(N + 1, 0), pcount(N + 1, 0);
   for (int p = 0; p < np; ++p) {
     const ProbPlan& P = B.probs[p];
-    const double c = step_cost(P.d.nm, P.nch);
     for (long long t = 0; t < P.sched.ntask(); ++t) {
       const int* r = &P.sched.rec[t * MSB_TASK_INTS];
       const long long g = first[p] + t;
       T[g].prob = p;
-      const int w = r[TK_X1] - r[TK_X0], h = r[TK_Y1] - r[TK_Y0], nz = r[TK_Z1] - r[TK_Z0];
-      T[g].dur = (float)(c * (nz + w + h - 2));
-      T[g].plane_delay = (float)(c * (w + h - 1));
+      double dur, pd;
+      task_times(P, r, &dur, &pd);
+      T[g].dur = (float)dur;
+      T[g].plane_delay = (float)pd;
       int n = 0;
       for (int k = TK_DEP_X; k <= TK_DEP_VO; ++k)
         if (r[k] >= 0) {
@@ -489,17 +578,22 @@ int simulate_and_order(BatchImpl& B) {
   return MSB_OK;
 }
 
-// Classes from the problems' (nm, nch) and the chosen tile per (nm, nch).
-void make_classes(BatchImpl& B, const std::map<std::pair<int, int>, bool>& tile24) {
+// How a batch is cut: on a device for the row kernel (`rows` gives a moment
+// count's rows per pipeline; 0 or absent: the rule's choice per problem),
+// else (host-only plans) in tiles of 4 x 2, or 2 x 4 where `tile24` says so.
+struct Shape {
+  bool device = false;
+  std::map<int, int> rows;
+  std::map<int, bool> tile24;
+};
+
+// Classes from the problems' moment counts and angle tiles.
+void make_classes(BatchImpl& B) {
   std::map<int, int> kind_to_cls;
   B.classes.clear();
   std::map<int, double> work;
   for (auto& p : B.probs) {
-    auto it = tile24.find({p.d.nm, p.nch});
-    const bool t24 = it != tile24.end() && it->second;
-    p.kind = batch_kind(p.d.nm, p.nch, t24);
-    p.tx = t24 ? 2 : 4;
-    p.ty = t24 ? 4 : 2;
+    p.kind = batch_kind(p.d.nm, p.nt);
     work[p.kind] += p.work;
   }
   // classes in increasing kind order: the kernel visits the kinds in that order
@@ -516,14 +610,13 @@ void make_classes(BatchImpl& B, const std::map<std::pair<int, int>, bool>& tile2
     c.nm = p.d.nm;
     c.nch = p.nch;
     c.tx = p.tx;
-    c.ty = p.ty;
+    c.ty = p.rw ? 2 : p.ty;  // row kernel: its smallest pipeline
   }
 }
 
 // Plans every problem, then the arena (scratch_bytes, or all the problems'
 // scratch capped at `cap`) and the task table.
-int plan_batch(BatchImpl& B, const msb_problem* probs, int n, const std::map<std::pair<int, int>, bool>& tile24,
-               size_t scratch_bytes, size_t cap) {
+int plan_batch(BatchImpl& B, const msb_problem* probs, int n, const Shape& shape, size_t scratch_bytes, size_t cap) {
   // one entry per 32-angle pass of every problem
   B.probs.clear();
   B.nuser = n;
@@ -531,8 +624,15 @@ int plan_batch(BatchImpl& B, const msb_problem* probs, int n, const std::map<std
   for (int i = 0; i < n; ++i) {
     const int npass = (probs[i].na + 31) / 32;
     first_entry[i] = (int)B.probs.size();
-    auto it = tile24.find({probs[i].nm, 1});
-    const bool t24 = it != tile24.end() && it->second;
+    auto it = shape.tile24.find(probs[i].nm);
+    const bool t24 = it != shape.tile24.end() && it->second;
+    int rw = 0;
+    if (shape.device) {
+      auto ir = shape.rows.find(probs[i].nm);
+      rw = ir != shape.rows.end() ? ir->second : 0;
+      // other problems fill the CTAs: no least number of tasks
+      if (!rw) rw = pick_rows(probs[i].ncell_x, probs[i].ncell_y, (probs[i].ne + 1) / 2, 0);
+    }
     for (int c = 0; c < npass; ++c) {
       ProbPlan e;
       e.d = probs[i];
@@ -543,8 +643,10 @@ int plan_batch(BatchImpl& B, const msb_problem* probs, int n, const std::map<std
       e.nac = std::min(32, probs[i].na - 32 * c);
       e.prev = c > 0 ? (int)B.probs.size() - 1 : -1;
       e.nch = 1;
+      e.rw = rw;
+      e.nt = shape.device ? std::min(4, (probs[i].na + 7) / 8) : 4;
       e.tx = t24 ? 2 : 4;
-      e.ty = t24 ? 4 : 2;
+      e.ty = rw ? rw : t24 ? 4 : 2;
       if (c > 0) B.probs.back().next = (int)B.probs.size();
       B.probs.push_back(e);
     }
@@ -573,7 +675,7 @@ int plan_batch(BatchImpl& B, const msb_problem* probs, int n, const std::map<std
       e.scratch = f.scratch;
       e.work = f.work;
     }
-  make_classes(B, tile24);
+  make_classes(B);
   if ((int)B.classes.size() > kMaxBatchClasses) return set_error(MSB_ERR_ARG, "batch: too many classes");
   size_t need = 0;
   for (auto& p : B.probs)
@@ -596,15 +698,14 @@ int setup_kernel(int* nsm) {
   int rc, dev = 0;
   if ((rc = cuda_check(cudaGetDevice(&dev), "cudaGetDevice"))) return rc;
   if ((rc = cuda_check(cudaDeviceGetAttribute(&sm, cudaDevAttrMultiProcessorCount, dev), "SM count"))) return rc;
-  constexpr size_t smem = fp64_batch_smem<kBatchStages>();
-  static_assert(smem <= 227 * 1024 - 1024, "shared memory budget of the batched kernel");
+  constexpr size_t smem = row_batch_smem();
   if (!done) {
-    if ((rc = cuda_check(cudaFuncSetAttribute(sweep_fp64_batch_kernel<kBatchStages>,
+    if ((rc = cuda_check(cudaFuncSetAttribute(sweep_fp64_row_batch_kernel,
                                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
                          "cudaFuncSetAttribute (batch)")))
       return rc;
     int occ = 0;
-    if ((rc = cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, sweep_fp64_batch_kernel<kBatchStages>,
+    if ((rc = cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, sweep_fp64_row_batch_kernel,
                                                                        384, smem),
                          "occupancy (batch)")))
       return rc;
@@ -643,6 +744,7 @@ int upload_batch(BatchImpl& B) {
     q.ngp = P.ngp;
     q.ia_base = P.a0;
     q.vo_add = P.pass > 0 ? 1 : 0;
+    q.rw = (signed char)P.rw;
     q.ie_base = 0;
   }
   if ((rc = upload(&B.d_tasks, B.rec, "batch tasks"))) return rc;
@@ -690,7 +792,7 @@ int enqueue_sweep(BatchImpl& B, int dir, cudaStream_t st) {
   if ((rc = cuda_check(cudaMemsetAsync(B.d_sync, 0, B.sync_ints * sizeof(int), st), "reset batch sync"))) return rc;
   const Fp64Batch P = launch_params(B, dir);
   const int grid = (int)std::min<long long>(B.ntask, (long long)B.nsm);
-  sweep_fp64_batch_kernel<kBatchStages><<<grid, 384, fp64_batch_smem<kBatchStages>(), st>>>(P);
+  sweep_fp64_row_batch_kernel<<<grid, 384, row_batch_smem(), st>>>(P);
   return cuda_check(cudaGetLastError(), "batched sweep launch");
 }
 
@@ -710,13 +812,13 @@ int sync_status(BatchImpl& B, cudaStream_t st) {
   return MSB_OK;
 }
 
-// Times both tile shapes on the median problem of each nm group (every
-// entry sweeps one 32-angle chunk) and returns the faster shape per group.  The trial sweeps write that problem's
-// vo array (the batch's own sweeps overwrite it later).
-int autotune(const msb_problem* probs, int n, int nsm, size_t arena, std::map<std::pair<int, int>, bool>* tile24,
-             double* tune_ms) {
-  std::map<std::pair<int, int>, std::vector<int>> groups;
-  for (int i = 0; i < n; ++i) groups[{probs[i].nm, 1}].push_back(i);
+// Times the row kernel with the rule's and with every fixed number of rows
+// per pipeline on the median problem of each moment count and returns the
+// fastest choice per count (0: the rule's).  The trial sweeps write that
+// problem's vo array (the batch's own sweeps overwrite it later).
+int autotune(const msb_problem* probs, int n, int nsm, size_t arena, std::map<int, int>* rows, double* tune_ms) {
+  std::map<int, std::vector<int>> groups;
+  for (int i = 0; i < n; ++i) groups[probs[i].nm].push_back(i);
   cudaStream_t st = nullptr;
   int rc = cuda_check(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking), "autotune stream");
   if (rc) return rc;
@@ -733,11 +835,14 @@ int autotune(const msb_problem* probs, int n, int nsm, size_t arena, std::map<st
     std::sort(v.begin(), v.end(), [&](int a, int b) { return cells(a) < cells(b); });
     const int rep = v[v.size() / 2];
     double best = 1e30;
-    bool best24 = false;
-    for (int t24 = 0; t24 < 2 && !rc; ++t24) {
+    int best_rw = 0;
+    for (int rw : {0, 8, 4, 2}) {
+      if (rc) break;
       BatchImpl T;
       T.nsm = nsm;
-      std::map<std::pair<int, int>, bool> choice{{g.first, t24 != 0}};
+      Shape choice;
+      choice.device = true;
+      choice.rows[g.first] = rw;
       if ((rc = plan_batch(T, &probs[rep], 1, choice, 0, arena))) break;
       if ((rc = upload_batch(T))) break;
       float ms = 0.f, acc = 0.f;
@@ -753,10 +858,10 @@ int autotune(const msb_problem* probs, int n, int nsm, size_t arena, std::map<st
       total += acc;
       if (!rc && acc < best) {
         best = acc;
-        best24 = t24 != 0;
+        best_rw = rw;
       }
     }
-    (*tile24)[g.first] = best24;
+    (*rows)[g.first] = best_rw;
     if (rc) break;
   }
   cudaEventDestroy(e0);
@@ -774,7 +879,6 @@ using msb::BatchImpl;
 struct msb_batch {
   BatchImpl impl;
   double tune_ms = 0.0;
-  int tile24[3][2] = {{0, 0}, {0, 0}, {0, 0}};
 };
 
 static int batch_build(msb_batch** out, const msb_problem* problems, int nproblem, int precision,
@@ -802,16 +906,13 @@ static int batch_build(msb_batch** out, const msb_problem* problems, int nproble
     if ((rc = msb::cuda_check(cudaMemGetInfo(&fr, &tot), "cudaMemGetInfo"))) return rc;
     cap = (size_t)(fr * 0.8);
   }
-  std::map<std::pair<int, int>, bool> tile24;
+  msb::Shape shape;
+  shape.device = true;
   if (autotune_flag && device) {
-    if ((rc = msb::autotune(problems, nproblem, B.nsm, scratch_bytes ? scratch_bytes : cap, &tile24, &b->tune_ms)))
+    if ((rc = msb::autotune(problems, nproblem, B.nsm, scratch_bytes ? scratch_bytes : cap, &shape.rows, &b->tune_ms)))
       return rc;
   }
-  for (auto& t : tile24) {
-    const int ni = t.first.first == 4 ? 0 : t.first.first == 8 ? 1 : 2;
-    b->tile24[ni][t.first.second - 1] = t.second ? 1 : 0;
-  }
-  if ((rc = msb::plan_batch(B, problems, nproblem, tile24, scratch_bytes, cap))) return rc;
+  if ((rc = msb::plan_batch(B, problems, nproblem, shape, scratch_bytes, cap))) return rc;
   if (device && (rc = msb::upload_batch(B))) return rc;
   *out = b.release();
   return MSB_OK;
@@ -835,10 +936,10 @@ extern "C" int msb_batch_plan(msb_batch** out, const msb_problem* problems, int 
   BatchImpl& B = b->impl;
   B.nsm = nsm;
   // bit (nm index) of the mask selects the 2 x 4 tile
-  std::map<std::pair<int, int>, bool> tile24;
+  msb::Shape shape;
   const int nms[3] = {4, 8, 16};
-  for (int k = 0; k < 3; ++k) tile24[{nms[k], 1}] = ((tile24_mask >> k) & 1) != 0;
-  if ((rc = msb::plan_batch(B, problems, nproblem, tile24, scratch_bytes, ~(size_t)0))) return rc;
+  for (int k = 0; k < 3; ++k) shape.tile24[nms[k]] = ((tile24_mask >> k) & 1) != 0;
+  if ((rc = msb::plan_batch(B, problems, nproblem, shape, scratch_bytes, ~(size_t)0))) return rc;
   *out = b.release();
   return MSB_OK;
 }
@@ -910,7 +1011,6 @@ extern "C" int msb_batch_info(const msb_batch* b, msb_batch_info_t* info) {
   memset(info, 0, sizeof *info);
   info->nproblem = B.nuser;
   info->ntask = B.ntask;
-  info->nclass = (int)B.classes.size();
   info->scratch_bytes = B.arena_bytes;
   size_t need = 0;
   for (auto& p : B.probs)
@@ -921,12 +1021,20 @@ extern "C" int msb_batch_info(const msb_batch* b, msb_batch_info_t* info) {
   info->sim_makespan = B.sim_makespan;
   info->sim_busy = B.sim_busy;
   info->tune_ms = b->tune_ms;
-  for (int c = 0; c < info->nclass && c < MSB_BATCH_MAX_CLASSES; ++c) {
-    info->class_nm[c] = B.classes[c].nm;
-    info->class_nch[c] = B.classes[c].nch;
-    info->class_tx[c] = B.classes[c].tx;
-    info->class_ty[c] = B.classes[c].ty;
-    info->class_ntask[c] = B.classes[c].ntask;
+  // the bodies of one moment count count as one class
+  info->nclass = 0;
+  for (const auto& k : B.classes) {
+    const int c = info->nclass;
+    if (c > 0 && info->class_nm[c - 1] == k.nm) {
+      info->class_ntask[c - 1] += k.ntask;
+      continue;
+    }
+    info->class_nm[c] = k.nm;
+    info->class_nch[c] = k.nch;
+    info->class_tx[c] = k.tx;
+    info->class_ty[c] = k.ty;
+    info->class_ntask[c] = k.ntask;
+    ++info->nclass;
   }
   return MSB_OK;
 }

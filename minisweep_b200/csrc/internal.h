@@ -78,6 +78,10 @@ int build_schedule(int nx, int ny, int nz, int ngp, int tx, int ty, int gp_block
 // about `window` tasks.
 int pick_gp_block(int nx, int ny, int ngp, int tx, int ty, int window);
 
+// Rows per pipeline of the row kernel (8, 4 or 2; a task then covers 1, 2 or 4
+// group pairs).  Fewer than 8 only with at least min_tasks tasks in a phase.
+int pick_rows(int nx, int ny, int ngp, int min_tasks);
+
 // ------------------------------------------------------- KBA decomposition
 // One slab of a decomposed sweep: one octant over the process's whole x-y
 // extent and the z-planes [z0, z1).  The edge flags say where the slab's

@@ -263,4 +263,22 @@ int pick_gp_block(int nx, int ny, int ngp, int tx, int ty, int window) {
   return b;
 }
 
+// 8 rows in one pipeline move the fewest y faces and leave the most CTAs to a
+// phase; where a region's rows leave many of the 8 warps idle and there are
+// tasks enough all the same, shorter pipelines share the CTA between group
+// pairs.  Measured, ms per sweep with 8, 4, 2 rows:
+//   64 x 64 x 64, ne 64   57.3  60    63.0     48 x 20 x 48, ne 32   7.29  6.43  6.45
+//   24 x 24 x 24, ne 8    0.78  0.85  0.97     40 x 6 x 40, ne 64    4.30  2.99  3.13
+//   10 x 10 x 10, ne 30   0.31  0.36  0.36     20 x 4 x 6, ne 64     0.42  0.35  0.33
+int pick_rows(int nx, int ny, int ngp, int min_tasks) {
+  const int hx = (nx + 1) / 2, h0 = (ny + 1) / 2, h1 = ny / 2;
+  if (8LL * ceil_div(hx, 4) * ceil_div(h0, 8) * ngp < min_tasks) return 8;
+  // rows x group pairs that a CTA's warps stand for, idle ones included
+  auto cost = [&](int rw, double faces) {
+    return (ceil_div(h0, rw) + ceil_div(h1, rw)) * rw * (double)(ceil_div(ngp, 8 / rw) * (8 / rw)) * faces;
+  };
+  const double c8 = cost(8, 1.15), c4 = cost(4, 1.05), c2 = cost(2, 1.45);
+  return c8 <= c4 && c8 <= c2 ? 8 : c4 <= c2 ? 4 : 2;
+}
+
 }  // namespace msb

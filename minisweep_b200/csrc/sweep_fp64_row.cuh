@@ -82,7 +82,7 @@ struct RowCfg {
 // A posted task: the table's record, where it starts in the CTA's count of
 // planes, and its problem.
 struct RowRec {
-  int oct, gp, x0, x1, y0, y1, z0, z1, flags, depx, depy, task, stop, plane0, prob, pad;
+  int oct, gp, x0, x1, y0, y1, z0, z1, flags, depx, depy, task, stop, plane0, prob, rw;
   Fp64Prob q;
 };
 static_assert(sizeof(RowRec) <= 24 * sizeof(double), "task record size");
@@ -368,6 +368,7 @@ __device__ __forceinline__ void row_tasker(const PP& P, int cls, double* smem) {
       rec->z0 = r[TK_Z0]; rec->z1 = r[TK_Z1];
       rec->flags = r[TK_FLAGS]; rec->depx = depx; rec->depy = depy;
       rec->task = t; rec->stop = 0; rec->plane0 = plane0[0]; rec->prob = prob;
+      rec->rw = Q.rw;
       rec->q = Q;
     }
     __syncwarp();
@@ -377,7 +378,7 @@ __device__ __forceinline__ void row_tasker(const PP& P, int cls, double* smem) {
 }
 
 template <int NM_, int NT, bool BATCH, class PP>
-__device__ __forceinline__ void row_fetcher(const PP& P, int rw, double* smem) {
+__device__ __forceinline__ void row_fetcher(const PP& P, double* smem) {
   using C = RowCfg<NM_, NT>;
   constexpr int E = C::E, DY = C::DY, R = C::R;
   const int lane = threadIdx.x & 31;
@@ -386,9 +387,8 @@ __device__ __forceinline__ void row_fetcher(const PP& P, int rw, double* smem) {
   const int* const progress = sync + SY_PROGRESS;
   uint64_t* const bars = reinterpret_cast<uint64_t*>(smem + C::SM_BAR);
 
-  const bool is_x = lane < R, is_y = lane >= R && lane < R + R / rw;
-  const int wrp = is_x ? lane : is_y ? (lane - R) * rw : 0;  // the compute warp this lane feeds
-  const int pipe = wrp / rw, row = wrp % rw;
+  const bool is_x = lane < R, is_y = lane >= R && lane < 2 * R;
+  const int wrp = lane % R;  // the compute warp this lane feeds
   const int depth = is_x ? 1 : DY;
   uint64_t* const full = is_x ? bars + wrp : bars + 2 * R + wrp * DY;
   uint64_t* const empty = full + (is_x ? R : R * DY);
@@ -398,10 +398,12 @@ __device__ __forceinline__ void row_fetcher(const PP& P, int rw, double* smem) {
   int k = 0;           // task
   int a = 0, c = 0;    // next face: position in the row (y), plane
   int w = 0, nzr = 0, dep = -1;
-  int F = 0;           // faces issued
+  int F = 0;           // faces the ring has taken
+  int own[2] = {0, 0}, prev[2] = {0, 0};  // those this lane copied itself: its last run, the one before
   int seen = 0;        // upwind planes seen complete
   long long t0 = 0;    // start of the present wait for the upwind tile
-  bool fail = false;
+  bool fail = false, handed = false;  // handed: the row before filled the ring since this lane last did
+  int plane0 = 0;
   const char* src = nullptr;
   long long fa = 0, fc = 0;  // byte strides
   for (;;) {
@@ -413,8 +415,15 @@ __device__ __forceinline__ void row_fetcher(const PP& P, int rw, double* smem) {
         live = false;
       } else {
         const Fp64Prob& Q = rec.q;
-        const int oct = rec.oct, gp = rec.gp * (R / rw) + pipe, flags = rec.flags;
-        if (row >= rec.y1 - rec.y0 || gp >= Q.ngp || !(flags & (is_x ? TF_X_IN : TF_Y_IN))) {
+        const int row = wrp % rec.rw, gp = rec.gp * (R / rec.rw) + wrp / rec.rw;
+        const int oct = rec.oct, flags = rec.flags;
+        const bool runs = row < rec.y1 - rec.y0 && gp < Q.ngp;  // the warp takes part in the task
+        if (!runs || (is_x ? !(flags & TF_X_IN) : row > 0 || !(flags & TF_Y_IN))) {
+          // the row before it fills the warp's y ring in this task
+          if (runs && is_y && row > 0) {
+            F += (rec.x1 - rec.x0) * (rec.z1 - rec.z0);
+            handed = true;
+          }
           ++k;
         } else {
           have = true;
@@ -423,6 +432,10 @@ __device__ __forceinline__ void row_fetcher(const PP& P, int rw, double* smem) {
           nzr = rec.z1 - rec.z0;
           a = c = 0;
           seen = 0;
+          prev[0] = own[0];
+          prev[1] = own[1];
+          own[0] = F;
+          plane0 = rec.plane0;
           const int ix = dx > 0 ? rec.x0 : rec.x1 - 1, iz = dz > 0 ? rec.z0 : rec.z1 - 1;
           const int iy = dy > 0 ? rec.y0 + row : rec.y1 - 1 - row;
           const long long ent = (long long)oct * Q.ngp + gp;
@@ -436,7 +449,10 @@ __device__ __forceinline__ void row_fetcher(const PP& P, int rw, double* smem) {
       }
     }
     if (live && have) {
-      bool go = F < depth || mbar_test_wait(&empty[F % depth], (uint32_t)((F / depth + 1) & 1));
+      // A ring that changes its producer may be many phases behind F, where
+      // the parity says nothing: first let the warp finish the earlier tasks.
+      if (handed && ld_acquire_cta(cnt + RC_PLANES + wrp) >= plane0) handed = false;
+      bool go = !handed && (F < depth || mbar_test_wait(&empty[F % depth], (uint32_t)((F / depth + 1) & 1)));
       if (go && dep >= 0 && seen < c + 1) {
         seen = ld_acquire(progress + dep);
         if (seen < c + 1) {
@@ -459,7 +475,7 @@ __device__ __forceinline__ void row_fetcher(const PP& P, int rw, double* smem) {
         uint64_t* const bar = &full[F % depth];
         mbar_arrive_expect_tx(bar, E * 8);
         bulk_g2s(dst + (F % depth) * E, src, E * 8, bar);
-        ++F;
+        own[1] = ++F;
         src += fa;
         if (++a == w) {
           a = 0;
@@ -479,12 +495,19 @@ __device__ __forceinline__ void row_fetcher(const PP& P, int rw, double* smem) {
     if (!__any_sync(0xffffffffu, moved)) __nanosleep(100);
     __syncwarp();
   }
-  // the copies of this lane land before the shared memory is reused or
-  // released (microseconds; the bound is 1 ms)
-  const long long t1 = global_ns();
-  for (int n = max(0, F - depth); n < F; ++n)
-    while (!mbar_test_wait(&full[n % depth], (uint32_t)((n / depth) & 1)) && global_ns() - t1 < 1000000) {
+  __syncwarp();
+  // After an early end the compute warps may not have waited for every copy:
+  // let them land before the shared memory is reused or released
+  // (microseconds; the bound is 1 ms).
+  if (ld_volatile(cnt + RC_QUIT) != 0) {
+    const long long t1 = global_ns();
+    for (int i = 0; i < 2; ++i) {
+      const int lo = i ? own[0] : prev[0], hi = i ? own[1] : prev[1];
+      for (int n = max(lo, hi - depth); n < hi; ++n)
+        while (!mbar_test_wait(&full[n % depth], (uint32_t)((n / depth) & 1)) && global_ns() - t1 < 1000000) {
+        }
     }
+  }
   __syncwarp();
 }
 
@@ -539,14 +562,13 @@ __device__ __forceinline__ void row_publisher(const PP& P, double* smem) {
   }
 }
 
-// One compute warp: row `warp % rw` of pipeline `warp / rw`.
-template <int NM_, int NT, class PP>
-__device__ __forceinline__ void row_compute(const PP& P, int rw, double* smem) {
+// One compute warp: row `warp % rw` of pipeline `warp / rw` of each task.
+template <int NM_, int NT, bool BATCH, class PP>
+__device__ __forceinline__ void row_compute(const PP& P, double* smem) {
   using C = RowCfg<NM_, NT>;
   constexpr int E = C::E, VSZ = C::VSZ, W = C::W, D = C::D, DY = C::DY, R = C::R, KS = C::KS, MT = C::MT;
   const int lane = threadIdx.x & 31, warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
   const int q = lane >> 2, r = lane & 3;
-  const int row = warp % rw, pipe = warp / rw;
   int* const cnt = reinterpret_cast<int*>(smem + C::SM_CNT);
   // shared-memory addresses of this warp's barriers, rings and face slots
   const uint32_t sb = smem_u32(smem);
@@ -564,15 +586,35 @@ __device__ __forceinline__ void row_compute(const PP& P, int rw, double* smem) {
   for (int i = 0; i < 2; ++i) wz[i] = 1.0 / 4.0 - 1.0 / (double)(1 << (2 * r + i));
 
   uint32_t x_ph = 0;                              // phase of the entering x face
-  uint32_t yi = 0, yi_ph = 0, yo = 0, yo_ph = 1;  // y rings: positions and phases
+  bool handed = false;           // the fetcher filled the next warp's ring since this warp last did
+  uint32_t n_in = 0, n_out = 0;  // y faces that passed through this warp's ring and the next warp's, earlier tasks
   for (int k = 0;; ++k) {
     if (!row_wait_count(cnt + RC_POSTED, k + 1, cnt, P.sy, 64)) return;
     const RowRec& rec = reinterpret_cast<const RowRec*>(smem + C::SM_REC)[k % C::NREC];
     if (rec.stop) return;
-    const int oct = rec.oct, flags = rec.flags, gp = rec.gp * (R / rw) + pipe;
+    const int oct = rec.oct, flags = rec.flags;
+    int rw;
+    if constexpr (BATCH) rw = rec.rw; else rw = P.pr.rw;
+    const int row = warp % rw, gp = rec.gp * (R / rw) + warp / rw;
     const Fp64Prob& Q = rec.q;
     const int w = rec.x1 - rec.x0, h = rec.y1 - rec.y0, nzr = rec.z1 - rec.z0;
-    if (row >= h || gp >= Q.ngp) {
+    const bool runs = row < h && gp < Q.ngp;
+    const bool y_feed = runs && (row > 0 || (flags & TF_Y_IN));  // the y face comes through the ring
+    const bool y_pass = runs && row + 1 < min(h, rw);            // ... and goes on through the next one
+    // ring positions and phases (an empty slot's phase lags by one)
+    uint32_t yi = n_in % DY, yi_ph = (n_in / DY) & 1, yo = n_out % DY, yo_ph = (n_out / DY + 1) & 1;
+    if (y_feed) n_in += w * nzr;
+    // the next warp's ring also takes faces where that warp begins a pipeline
+    // and the fetcher feeds it
+    const int row2 = (warp + 1) % rw, gp2 = rec.gp * (R / rw) + (warp + 1) / rw;
+    const bool fetched = row2 == 0 && gp2 < Q.ngp && (flags & TF_Y_IN);
+    if (y_pass || fetched) n_out += w * nzr;
+    if (y_pass && handed) {  // as in the fetcher: a ring that changes its producer
+      if (!row_wait_count(cnt + RC_PLANES + warp + 1, rec.plane0, cnt, P.sy, 64)) return;
+      handed = false;
+    }
+    if (fetched) handed = true;
+    if (!runs) {
       __syncwarp();
       if (lane == 0) st_release_cta(cnt + RC_PLANES + warp, rec.plane0 + nzr);
       continue;
@@ -586,8 +628,6 @@ __device__ __forceinline__ void row_compute(const PP& P, int rw, double* smem) {
     const double so = (double)(1 + oct);
     const double so_r = 1.0 / so;  // rounded, as the reference's 1/(1+octant)
     int sp0 = ix0 + 3 * iy + 7 * iz0 + 2 + Q.sp_off;  // log2 s_space of the row's first cell, mod 4
-    const bool y_feed = row > 0 || (flags & TF_Y_IN);       // the y face comes through the ring
-    const bool y_pass = row + 1 < h;                        // ... and goes on through the next one
     const bool y_out = !y_pass && (flags & TF_Y_OUT);
     const bool x_in = (flags & TF_X_IN) != 0, z_in = (flags & TF_Z_IN) != 0;
     const bool x_out = (flags & TF_X_OUT) != 0, z_out = (flags & TF_Z_OUT) != 0;
@@ -857,22 +897,29 @@ __device__ __forceinline__ void row_setup(double* smem, bool init) {
   }
 }
 
+// The producer warps of one body.
+template <int NM_, int NT, bool BATCH, class PP>
+__device__ __forceinline__ void row_producers(const PP& P, int cls, double* smem) {
+  using C = RowCfg<NM_, NT>;
+  const int warp = threadIdx.x >> 5;
+  if (warp == C::R) row_tasker<NM_, NT, BATCH>(P, cls, smem);
+  else if (warp == C::R + 1) row_fetcher<NM_, NT, BATCH>(P, smem);
+  else if (warp == C::R + 2) row_publisher<NM_, NT, BATCH>(P, smem);
+}
+
 template <int NM_, int NT>
 __global__ void __launch_bounds__(RowCfg<NM_, NT>::NTH, 1) sweep_fp64_row_kernel(const Fp64Params P) {
   using C = RowCfg<NM_, NT>;
   extern __shared__ __align__(128) double smem[];
   if (threadIdx.x == 0) row_setup<NM_, NT>(smem, true);
   __syncthreads();
-  const int warp = threadIdx.x >> 5;
   // 384 threads x 168 registers: 8 warps x 32 x 208 + 4 x 32 x 80
-  if (warp >= C::R) {
+  if ((threadIdx.x >> 5) >= C::R) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(80));
-    if (warp == C::R) row_tasker<NM_, NT, false>(P, 0, smem);
-    else if (warp == C::R + 1) row_fetcher<NM_, NT, false>(P, P.rw, smem);
-    else if (warp == C::R + 2) row_publisher<NM_, NT, false>(P, smem);
+    row_producers<NM_, NT, false>(P, 0, smem);
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(208));
-    row_compute<NM_, NT>(P, P.rw, smem);
+    row_compute<NM_, NT, false>(P, smem);
   }
 }
 

@@ -64,7 +64,7 @@ struct Fp64Prob {
   signed char l2_hints;  // nonzero: faces written evict_last, state and consumed faces evict_first (chained kernel)
   signed char sp_off;    // (ix_base + 3 iy_base) & 3 of a process's subdomain (KBA decomposition): the space
                          // factor (quantities_testing_kernels.h:97-126) takes global coordinates
-  signed char pad_;
+  signed char rw;        // rows per pipeline of the row kernel (8, 4 or 2)
   int a_stride;  // angles per octant row of afm / mfa (0: na); afm and mfa then point at the pass's first
                  // angle of the caller's full matrices (a batch's angle passes read them in place)
 };
@@ -76,7 +76,6 @@ struct Fp64Params {
   const int* tasks;
   long long ntask;
   SyncArgs sy;
-  int rw;  // row kernel: rows per pipeline (8, 4 or 2)
 };
 
 // Many problems per launch.  Tasks of all problems share one table with
@@ -155,42 +154,15 @@ struct Fp64Cfg {
   static constexpr int SM_MAT = SM_STAGE + NS * STAGE;  // [2][MAT]
   static constexpr int SM_BAR = SM_MAT + 2 * MAT;       // full[NS], done[NS], freed[NS]
   static constexpr int SM_FINAL = SM_BAR + 3 * NS;      // loader -> publisher: steps issued (int)
-  static constexpr int SM_PROB = SM_FINAL + 1;          // batched: Fp64Prob of the task in each mat buffer
-  static constexpr size_t smem_bytes() { return sizeof(double) * (size_t)SM_PROB; }
-  // batched: two problem records, then the problem whose predecessors the loader last saw complete (int)
-  static constexpr size_t smem_bytes_batch() { return sizeof(double) * (size_t)SM_PROB + 2 * sizeof(Fp64Prob) + 16; }
+  static constexpr int SM_END = SM_FINAL + 1;
+  static constexpr size_t smem_bytes() { return sizeof(double) * (size_t)SM_END; }
 };
 
-// Shared-memory barriers of one body: set up before its first stage, and
-// invalidated before another body reuses the memory.
-template <int NM_, int NCH, int TX, int TY, int NS>
-__device__ __forceinline__ void fp64_barriers(bool init) {
-  using C = Fp64Cfg<NM_, NCH, TX, TY, NS>;
-  extern __shared__ __align__(128) double smem[];
-  uint64_t* const bars = reinterpret_cast<uint64_t*>(smem + C::SM_BAR);
-  if (init) {
-    for (int i = 0; i < NS; ++i) {
-      mbar_init(&bars[i], 1);            // full: the loader's arrive.expect_tx (header + face copies)
-      mbar_init(&bars[NS + i], 1);       // done: compute warp 0, after the compute warps' step barrier
-      mbar_init(&bars[2 * NS + i], 1);   // freed: the publisher
-    }
-    *reinterpret_cast<volatile int*>(smem + C::SM_FINAL) = -1;
-    reinterpret_cast<volatile int*>(smem + C::SM_FINAL)[1] = 0;  // compute warps' quit flag
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  } else {
-    for (int i = 0; i < 3 * NS; ++i) mbar_inval(&bars[i]);
-  }
-}
-
-// The sweep of one class of tasks by one CTA.  ROLE 0: the whole CTA (sets
-// up its barriers, then splits into the producer warpgroup and the compute
-// warps, moving registers from the first to the second); ROLE 1: the
-// producer warps only; ROLE 2: the compute warps only (a batched kernel
-// splits the roles once and sets up the barriers of each class itself).
-// BATCH: P is an Fp64Batch and `cls` the class whose table range this call
-// works through; otherwise P is an Fp64Params.
-template <int NM_, int NCH, int TX, int TY, int NS, bool PIPE_T1, bool BATCH, int ROLE, class PP>
-__device__ __forceinline__ void fp64_body(const PP& P, int cls) {
+// The sweep by one CTA: sets up the barriers, then splits into the producer
+// warpgroup and the compute warps, moving registers from the first to the
+// second.
+template <int NM_, int NCH, int TX, int TY, int NS, bool PIPE_T1>
+__global__ void __launch_bounds__((TX * TY + 4) * 32, 1) sweep_fp64_kernel(const Fp64Params P) {
   using C = Fp64Cfg<NM_, NCH, TX, TY, NS>;
   constexpr int KS = C::KS, MT = C::MT, NW = C::NW, ENT = C::ENT, VSZ = C::VSZ;
   static_assert(NM_ % 4 == 0 && NM_ <= 16, "NM must be 4, 8 or 16");
@@ -203,31 +175,32 @@ __device__ __forceinline__ void fp64_body(const PP& P, int cls) {
   uint64_t* const done = full + NS;
   uint64_t* const freed = done + NS;  // publisher consumed the step: loader may refill the stage
 
-  Fp64Prob* const s_prob = reinterpret_cast<Fp64Prob*>(smem + C::SM_PROB);  // BATCH only
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int* const sync = P.sy.sync;
   int* const progress = sync + SY_PROGRESS;
   // loader <-> publisher hand-off: total steps issued, once the loader stops (-1 before)
   volatile int& s_final = *reinterpret_cast<volatile int*>(smem + C::SM_FINAL);
 
-  if constexpr (ROLE == 0) {
-    if (threadIdx.x == 0) fp64_barriers<NM_, NCH, TX, TY, NS>(true);
-    __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < NS; ++i) {
+      mbar_init(&full[i], 1);   // the loader's arrive.expect_tx (header + face copies)
+      mbar_init(&done[i], 1);   // compute warp 0, after the compute warps' step barrier
+      mbar_init(&freed[i], 1);  // the publisher
+    }
+    s_final = -1;
+    reinterpret_cast<volatile int*>(smem + C::SM_FINAL)[1] = 0;  // compute warps' quit flag
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  __syncthreads();
 
-  if (ROLE == 1 || (ROLE == 0 && warp >= NW)) {
+  if (warp >= NW) {
     // ====================================================== producer warpgroup
-    if constexpr (C::REBALANCE && ROLE == 0) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(C::REG_PRODUCER));
+    if constexpr (C::REBALANCE) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(C::REG_PRODUCER));
     if (warp == NW) {
       // ------------------------------------------------------------ loader
       long long g_load = 0;
       long long last_step[2] = {-1, -1};  // last global step of the task using mat buffer 0/1
       int ntask_seen = 0;
-      // BATCH: the problem whose predecessors were last seen complete (kept
-      // in shared memory: the producer warps' registers are all in use)
-      volatile int* const preds_done_for = reinterpret_cast<volatile int*>(s_prob + 2);
-      if (BATCH && lane == 0) *preds_done_for = -1;
-      __syncwarp();
       bool failed = false;
 
       // Steps up to freed_upto have been consumed by the publisher.  Waiting
@@ -260,13 +233,8 @@ __device__ __forceinline__ void fp64_body(const PP& P, int cls) {
       auto grab = [&]() -> int {
         int t = -1;
         if (lane == 0 && ld_relaxed(&sync[SY_ABORT]) == 0) {
-          if constexpr (BATCH) {
-            const long long tt = atomicAdd(&sync[SY_CLASS0 + cls], 1);
-            t = tt < P.cls_ntask[cls] ? (int)(P.cls_base[cls] + tt) : -1;
-          } else {
-            const long long tt = atomicAdd(&sync[SY_COUNTER], 1);
-            t = tt < P.ntask ? (int)tt : -1;
-          }
+          const long long tt = atomicAdd(&sync[SY_COUNTER], 1);
+          t = tt < P.ntask ? (int)tt : -1;
         }
         return __shfl_sync(0xffffffffu, t, 0);
       };
@@ -289,31 +257,7 @@ __device__ __forceinline__ void fp64_body(const PP& P, int cls) {
         const int dx = (oct & 1) ? -1 : 1, dy = (oct & 2) ? -1 : 1, dz = (oct & 4) ? -1 : 1;
         const int depx = (mode & DM_X_PLANE) ? rec[TK_DEP_X] : -1;
         const int depy = (mode & DM_Y_PLANE) ? rec[TK_DEP_Y] : -1;
-        // the task's problem
-        Fp64Prob Q;
-        int prob = 0;
-        if constexpr (BATCH) {
-          prob = __ldg(&P.task_prob[t]);
-          Q = P.probs[prob];
-          if (P.dir) {
-            const double* a = Q.vi;
-            Q.vi = Q.vo;
-            Q.vo = const_cast<double*>(a);
-          }
-          // the face scratch is free once its previous users completed
-          // (completion is final: checked once per run of tasks of one problem)
-          if (prob != *preds_done_for) {
-            for (int k = __ldg(&P.pred_off[prob]), ke = __ldg(&P.pred_off[prob + 1]); k < ke && !failed; ++k) {
-              const int q2 = __ldg(&P.pred[k]);
-              if (wait_dep(&P.pdone[q2], __ldg(&P.prob_ntask[q2]), t) < 0) failed = true;
-            }
-            __syncwarp();
-            if (!failed && lane == 0) *preds_done_for = prob;
-            __syncwarp();
-          }
-        } else {
-          Q = P.pr;
-        }
+        const Fp64Prob& Q = P.pr;
         // cross-phase dependencies: whole task complete
         if (!failed && rec[TK_DEP_X] >= 0 && depx < 0 && wait_dep(&progress[rec[TK_DEP_X]], kComplete, t) < 0) failed = true;
         if (!failed && rec[TK_DEP_Y] >= 0 && depy < 0 && wait_dep(&progress[rec[TK_DEP_Y]], kComplete, t) < 0) failed = true;
@@ -336,9 +280,6 @@ __device__ __forceinline__ void fp64_body(const PP& P, int cls) {
           const int ia = 32 * ch + 8 * tt + 2 * (ln & 3) + i, im = 8 * mt + (ln >> 2);
           mat[NCH * KS * 4 * 32 + e] =
               (ia < Q.na && im < NM_) ? __ldg(&Q.mfa[im + (size_t)NM_ * (ia + as * oct)]) : 0.0;
-        }
-        if constexpr (BATCH) {
-          if (lane == 0) s_prob[mb] = Q;  // published to the compute warps with the task's first stage
         }
         __syncwarp();
         ++ntask_seen;
@@ -379,7 +320,7 @@ __device__ __forceinline__ void fp64_body(const PP& P, int cls) {
           if (lane == 0) {
             hdr->task = t; hdr->s = s; hdr->oct = oct; hdr->gp = gp;
             hdr->x0 = x0; hdr->x1 = x1; hdr->y0 = y0; hdr->y1 = y1; hdr->z0 = z0; hdr->z1 = z1;
-            hdr->flags = flags; hdr->mat = mb; hdr->stop = 0; hdr->pad1 = prob;
+            hdr->flags = flags; hdr->mat = mb; hdr->stop = 0;
             // progress this task reaches once step s is done (-2: nothing new)
             hdr->pad0 = s == nsteps - 1 ? kComplete : (s + 1 - (w + h - 2) > 0 ? s + 1 - (w + h - 2) : -2);
             mbar_arrive_expect_tx(&full[st], bytes);
@@ -458,22 +399,20 @@ __device__ __forceinline__ void fp64_body(const PP& P, int cls) {
           }
         }
         if (!ready) break;
-        int pend_task[2] = {-1, -1}, pend_val[2] = {-2, -2}, pend_prob[2] = {0, 0};
+        int pend_task[2] = {-1, -1}, pend_val[2] = {-2, -2};
         for (;;) {  // consume step G and any later steps already done
           const int st = (int)(G % NS);
           const StepHdr* hdr = reinterpret_cast<const StepHdr*>(stages + (size_t)st * C::STAGE + C::ST_HDR);
-          const int task = hdr->task, val = hdr->pad0, hprob = hdr->pad1;
+          const int task = hdr->task, val = hdr->pad0;
           __syncwarp();
           if (lane == 0) mbar_arrive(&freed[st]);
           if (val != -2) {
             if (pend_task[1] >= 0 && pend_task[1] != task) {
               pend_task[0] = pend_task[1];
               pend_val[0] = pend_val[1];
-              pend_prob[0] = pend_prob[1];
             }
             pend_task[1] = task;
             pend_val[1] = val;
-            pend_prob[1] = hprob;
           }
           ++G;
           // a task boundary ends a batch so older tasks are published first
@@ -487,22 +426,13 @@ __device__ __forceinline__ void fp64_body(const PP& P, int cls) {
           if (lane == 0) {
             if (pend_task[0] >= 0) st_release(&progress[pend_task[0]], pend_val[0]);
             if (pend_task[1] >= 0) st_release(&progress[pend_task[1]], pend_val[1]);
-            if constexpr (BATCH) {
-              // a problem is complete once all its tasks are: the last one
-              // stamps the time and releases its face scratch to later problems
-              for (int k = 0; k < 2; ++k)
-                if (pend_task[k] >= 0 && pend_val[k] == kComplete) {
-                  const int pr2 = pend_prob[k];
-                  if (atom_add_release(&P.pdone[pr2], 1) + 1 == __ldg(&P.prob_ntask[pr2])) P.ptime[pr2] = global_ns();
-                }
-            }
           }
         }
         t0 = global_ns();
       }
     }
   } else {
-  if constexpr (C::REBALANCE && ROLE == 0) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(C::REG_COMPUTE));
+  if constexpr (C::REBALANCE) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(C::REG_COMPUTE));
 
   // ================================================================ compute
   const int q = lane >> 2, r = lane & 3;
@@ -541,12 +471,7 @@ __device__ __forceinline__ void fp64_body(const PP& P, int cls) {
     const int oct = hdr0->oct, gp = hdr0->gp, flags = hdr0->flags;
     const int x0 = hdr0->x0, x1 = hdr0->x1, y0 = hdr0->y0, y1 = hdr0->y1, z0 = hdr0->z0, z1 = hdr0->z1;
     const double* mat = mats + hdr0->mat * C::MAT;
-    // the task's problem: the launch's own, or (batched) the loader's copy in
-    // shared memory, read where used rather than held in registers
-    Fp64Prob Qv;
-    const Fp64Prob* qp = &Qv;
-    if constexpr (BATCH) qp = s_prob + hdr0->mat; else Qv = P.pr;
-    const Fp64Prob& Q = *qp;
+    const Fp64Prob& Q = P.pr;
     const size_t slab = (size_t)NM_ * NU * Q.nx * Q.ny;  // one (iz, ie) layer of the state
     const int w = x1 - x0, h = y1 - y0, nzr = z1 - z0, nsteps = nzr + w + h - 2;
     const int dx = (oct & 1) ? -1 : 1, dy = (oct & 2) ? -1 : 1, dz = (oct & 4) ? -1 : 1;
@@ -801,100 +726,5 @@ __device__ __forceinline__ void fp64_body(const PP& P, int cls) {
   }
 }
 
-template <int NM_, int NCH, int TX, int TY, int NS, bool PIPE_T1>
-__global__ void __launch_bounds__((TX * TY + 4) * 32, 1) sweep_fp64_kernel(const Fp64Params P) {
-  fp64_body<NM_, NCH, TX, TY, NS, PIPE_T1, false, 0>(P, 0);
-}
-
-// Batched FP64 sweep: one class kind per (NM, angle chunks, tile shape), all
-// with 8 compute warps + the producer warpgroup (384 threads).  The CTAs work
-// through the classes in order; a CTA moves on when its class's table is
-// exhausted, so a task only ever waits on tasks that CTAs hold and advance.
-enum Fp64BatchKind {
-  BK_NM4_C1_42 = 0, BK_NM4_C1_24, BK_NM4_C2_42, BK_NM4_C2_24,
-  BK_NM8_C1_42, BK_NM8_C1_24, BK_NM8_C2_42, BK_NM8_C2_24,
-  BK_NM16_C1_42, BK_NM16_C1_24, BK_NM16_C2_42, BK_NM16_C2_24,
-  BK_COUNT
-};
-constexpr int batch_kind(int nm, int nch, bool tile24) {
-  return (nm == 4 ? 0 : nm == 8 ? 4 : 8) + (nch == 2 ? 2 : 0) + (tile24 ? 1 : 0);
-}
-
-// Every body kind of the batched kernel, in increasing kind order:
-// F(kind, NM, NCH, TX, TY).  A batch sweeps its problems in 32-angle
-// entries, so only the one-chunk bodies are compiled.
-#define MSB_FP64_BATCH_KINDS(F)                                                                   \
-  F(BK_NM4_C1_42, 4, 1, 4, 2) F(BK_NM4_C1_24, 4, 1, 2, 4) F(BK_NM8_C1_42, 8, 1, 4, 2)             \
-  F(BK_NM8_C1_24, 8, 1, 2, 4) F(BK_NM16_C1_42, 16, 1, 4, 2) F(BK_NM16_C1_24, 16, 1, 2, 4)
-
-// Between two classes: every warp of the CTA is done with the previous
-// class's stages (a barrier that warps reach from their own role's code, so
-// the non-aligned form), thread 0 swaps the barrier sets, and nobody starts
-// the new class before that.
-template <int NS>
-__device__ __forceinline__ void fp64_batch_switch(const Fp64Batch& P, int c) {
-  asm volatile("barrier.sync 0;" ::: "memory");
-  if (threadIdx.x == 0) {
-#define MSB_K(K, NM, NCH, TX, TY) \
-  case K: fp64_barriers<NM, NCH, TX, TY, NS>(init); break;
-    for (int k = 0; k < 2; ++k) {
-      const bool init = k == 1;
-      const int cc = init ? c : c - 1;
-      if (cc < 0 || cc >= P.nclass) continue;
-      switch (P.cls_kind[cc]) { MSB_FP64_BATCH_KINDS(MSB_K) default: break; }
-    }
-#undef MSB_K
-  }
-  asm volatile("barrier.sync 0;" ::: "memory");
-}
-
-// The classes of a launch come in increasing kind order (the host sorts
-// them so), and the kernel visits the kinds in that order, one straight-line
-// region per kind: compiled as separate regions (rather than the cases of a
-// switch) the bodies keep their register allocations apart.
-// Register split of the batched kernel (all class bodies in one kernel):
-// 200 / 96 (its producer code spills with the single-problem kernel's 80).
-constexpr int kBatchRegCompute = 200, kBatchRegProducer = 96;
-static_assert(8 * 32 * kBatchRegCompute + 4 * 32 * kBatchRegProducer <= 12 * 32 * 168, "batch register split");
-
-template <int NS>
-__global__ void __launch_bounds__(12 * 32, 1) sweep_fp64_batch_kernel(const Fp64Batch P) {
-  if (blockIdx.x == 0 && threadIdx.x == 0) P.ptime[P.nprob] = global_ns();
-  // the register split of the 8-compute-warp bodies, once for all classes
-  if ((threadIdx.x >> 5) >= 8) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kBatchRegProducer));
-    int c = 0;
-#define MSB_K(K, NM, NCH, TX, TY)                                 \
-  if (c < P.nclass && P.cls_kind[c] == K) {                       \
-    fp64_batch_switch<NS>(P, c);                                  \
-    fp64_body<NM, NCH, TX, TY, NS, false, true, 1>(P, c);         \
-    ++c;                                                          \
-  }
-    MSB_FP64_BATCH_KINDS(MSB_K)
-#undef MSB_K
-  } else {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kBatchRegCompute));
-    int c = 0;
-#define MSB_K(K, NM, NCH, TX, TY)                                 \
-  if (c < P.nclass && P.cls_kind[c] == K) {                       \
-    fp64_batch_switch<NS>(P, c);                                  \
-    fp64_body<NM, NCH, TX, TY, NS, false, true, 2>(P, c);         \
-    ++c;                                                          \
-  }
-    MSB_FP64_BATCH_KINDS(MSB_K)
-#undef MSB_K
-  }
-}
-
-// Dynamic shared memory of the batched kernel: the largest class body.
-template <int NS>
-constexpr size_t fp64_batch_smem() {
-  size_t m = 0;
-  const size_t v[] = {Fp64Cfg<4, 1, 4, 2, NS>::smem_bytes_batch(),  Fp64Cfg<4, 1, 2, 4, NS>::smem_bytes_batch(),
-                      Fp64Cfg<8, 1, 4, 2, NS>::smem_bytes_batch(),  Fp64Cfg<8, 1, 2, 4, NS>::smem_bytes_batch(),
-                      Fp64Cfg<16, 1, 4, 2, NS>::smem_bytes_batch(), Fp64Cfg<16, 1, 2, 4, NS>::smem_bytes_batch()};
-  for (size_t x : v) m = x > m ? x : m;
-  return m;
-}
 
 }  // namespace msb

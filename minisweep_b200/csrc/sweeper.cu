@@ -320,23 +320,6 @@ struct SweeperImpl {
 // ranges whose contributions add up in vo.
 static int pass_angles(const SweeperImpl& S) { return S.var.pass; }
 
-// Rows per pipeline of the row kernel.  8 rows in one pipeline move the fewest
-// y faces and leave the most CTAs to a phase; where a region's rows leave many
-// of the 8 warps idle and there are tasks enough for every CTA all the same
-// (4 rounds or more), shorter pipelines share the CTA between group pairs.
-// Measured, ms per sweep with 8, 4, 2 rows:
-//   64 x 64 x 64, ne 64   57.3  60    63.0     48 x 20 x 48, ne 32   7.29  6.43  6.45
-//   24 x 24 x 24, ne 8    0.78  0.85  0.97     40 x 6 x 40, ne 64    4.30  2.99  3.13
-//   10 x 10 x 10, ne 30   0.31  0.36  0.36     20 x 4 x 6, ne 64     0.42  0.35  0.33
-static int pick_rows(const Dimensions& d, int ngp, int nsm) {
-  const int hx = (d.ncell_x + 1) / 2, h0 = (d.ncell_y + 1) / 2, h1 = d.ncell_y / 2;
-  auto up = [](int n, int m) { return (n + m - 1) / m; };
-  if (8LL * up(hx, 4) * up(h0, 8) * ngp < 4LL * nsm) return 8;
-  auto cost = [&](int rw, double faces) { return (up(h0, rw) + up(h1, rw)) * rw * faces; };
-  const double c8 = cost(8, 1.15), c4 = cost(4, 1.05), c2 = cost(2, 1.45);
-  return c8 <= c4 && c8 <= c2 ? 8 : c4 <= c2 ? 4 : 2;
-}
-
 // Schedule, device task table and grid of one compiled tile shape, with a
 // window of `window` x SMs consecutive tasks between a tile and its downwind
 // neighbour in the table.
@@ -394,7 +377,7 @@ static int impl_create(SweeperImpl& S, const Dimensions& dims, int precision, in
   S.nsm = nsm;
   // no flag asks for a shape or a kernel: the row kernel
   if (precision == 0 && kernel == 0 && tile == 0 && angle_pass == 0 && !autotune)
-    S.var = pick_row(dims.nm, dims.na, pick_rows(dims, S.ngp, nsm));
+    S.var = pick_row(dims.nm, dims.na, pick_rows(dims.ncell_x, dims.ncell_y, S.ngp, 4 * nsm));
   if ((rc = setup_plan(S, S.var, S.window, S.sched, S.gp_block, S.d_tasks, S.grid))) return rc;
   long long ntask = S.sched.ntask();
   if (autotune) {
@@ -556,7 +539,7 @@ static int launch_fp64(SweeperImpl& S, const Variant& var, const int* d_tasks, l
     }
     if (var.rw) {
       const int b = (nac + 7) / 8 - 1;
-      P.rw = var.rw;
+      P.pr.rw = (signed char)var.rw;
       var.row_fn[b]<<<grid, var.threads, var.row_smem[b], stream>>>(P);
     } else {
       var.fn<<<grid, var.threads, var.smem, stream>>>(P);

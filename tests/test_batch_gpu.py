@@ -190,3 +190,20 @@ def test_batch_timeout_reports_and_recovers():
         b.sweep(0)
         b.sync()
     assert np.array_equal(D.vo[0].cpu().numpy(), single(probs[0], D.host_vi[0]))
+
+
+def test_batch_mixed_pipelines():
+    """Problems of one moment count whose region rows call for pipelines of 8,
+    4 and 2 rows, many of each, so that consecutive tasks of a CTA change the
+    pipeline height (and with it who fills a warp's ring of y faces)."""
+    W = []
+    for k in range(60):
+        ny, ne = [(16, 2), (5, 9), (4, 16), (9, 3), (3, 8), (12, 5)][k % 6]
+        W.append(dict(ncell_x=3 + k % 7, ncell_y=ny, ncell_z=2 + k % 5, ne=ne, na=32 if k % 4 else 16, nm=4))
+    D = Device(W)
+    with msb.Batch(D.descs) as b:
+        for _ in range(3):
+            b.sweep(0)
+        b.sync()
+    for i, p in enumerate(W):
+        assert np.array_equal(D.vo[i].cpu().numpy(), single(p, D.host_vi[i])), (i, p)
