@@ -71,7 +71,7 @@ __device__ __forceinline__ void row_batch_switch(const Fp64Batch& P, int c, doub
       if (cc < 0 || cc >= P.nclass) continue;
       switch (P.cls_kind[cc]) {
 #define MSB_K(NM, NT) \
-  case batch_kind(NM, NT): row_setup<NM, NT>(smem, init); break;
+  case batch_kind(NM, NT): row_setup<RowCfg<NM, NT>>(smem, init); break;
         MSB_ROW_BATCH_KINDS(MSB_K)
 #undef MSB_K
         default: break;
@@ -93,7 +93,7 @@ __global__ void __launch_bounds__(384, 1) sweep_fp64_row_batch_kernel(const Fp64
 #define MSB_K(NM, NT)                                              \
   if (c < P.nclass && P.cls_kind[c] == batch_kind(NM, NT)) {       \
     row_batch_switch(P, c, smem);                                  \
-    row_producers<NM, NT, true>(P, c, smem);                       \
+    row_producers<RowCfg<NM, NT>, true>(P, c, smem);                       \
     ++c;                                                           \
   }
     MSB_ROW_BATCH_KINDS(MSB_K)

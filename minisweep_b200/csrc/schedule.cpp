@@ -277,7 +277,7 @@ int pick_rows(int nx, int ny, int ngp, int min_tasks) {
   auto cost = [&](int rw, double faces) {
     return (ceil_div(h0, rw) + ceil_div(h1, rw)) * rw * (double)(ceil_div(ngp, 8 / rw) * (8 / rw)) * faces;
   };
-  const double c8 = cost(8, 1.15), c4 = cost(4, 1.05), c2 = cost(2, 1.45);
+  const double c8 = cost(8, 1.0), c4 = cost(4, 1.2), c2 = cost(2, 1.65);
   return c8 <= c4 && c8 <= c2 ? 8 : c4 <= c2 ? 4 : 2;
 }
 

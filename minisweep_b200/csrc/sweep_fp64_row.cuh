@@ -51,6 +51,12 @@
 
 namespace msb {
 
+// 8-byte asynchronous copy global -> shared, or zeros when !in
+__device__ __forceinline__ void cp_async8_zfill(void* dst, const void* src, bool in) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(in ? 8 : 0)
+               : "memory");
+}
+
 template <int NM_, int NT>
 struct RowCfg {
   static constexpr int W = 4, R = 8;          // cells per row, compute warps
@@ -77,6 +83,26 @@ struct RowCfg {
   static constexpr int SM_CNT = SM_REC + NREC * 24;     // counters (ints)
   static constexpr int SM_END = SM_CNT + 16;
   static constexpr size_t smem_bytes() { return sizeof(double) * (size_t)SM_END; }
+
+  // The octant's matrices in fragment order, zero beyond the last angle, by
+  // the 8-byte asynchronous copies of one warp.
+  static __device__ __forceinline__ void load_matrices(double* mat, const Fp64Prob& Q, int oct, int lane) {
+    const size_t as = Q.a_stride ? (size_t)Q.a_stride : (size_t)Q.na;
+#pragma unroll 4
+    for (int e = lane; e < KS * NT * 32; e += 32) {
+      const int tt = (e >> 5) % NT, ks = (e >> 5) / NT;
+      const int ia = 8 * tt + (lane >> 2), im = KS * (lane & 3) + ks;
+      const bool in = ia < Q.na;
+      cp_async8_zfill(&mat[e], &Q.afm[in ? ia + as * (im + (size_t)NM_ * oct) : 0], in);
+    }
+#pragma unroll 4
+    for (int e = lane; e < MT * NT * 2 * 32; e += 32) {
+      const int i = (e >> 5) & 1, tt = (e >> 6) % NT, mt = (e >> 6) / NT;
+      const int ia = 8 * tt + 2 * (lane & 3) + i, im = 8 * mt + (lane >> 2);
+      const bool in = ia < Q.na && im < NM_;
+      cp_async8_zfill(&mat[KS * NT * 32 + e], &Q.mfa[in ? im + (size_t)NM_ * (ia + as * oct) : 0], in);
+    }
+  }
 };
 
 // A posted task: the table's record, where it starts in the CTA's count of
@@ -104,11 +130,6 @@ __device__ __forceinline__ void st_release_cta(int* p, int v) {
   asm volatile("st.release.cta.shared::cta.s32 [%0], %1;" ::"r"(smem_u32(p)), "r"(v) : "memory");
 }
 __device__ __forceinline__ int ld_volatile(const int* p) { return *reinterpret_cast<const volatile int*>(p); }
-// 8-byte asynchronous copy global -> shared, or zeros when !in
-__device__ __forceinline__ void cp_async8_zfill(void* dst, const void* src, bool in) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(in ? 8 : 0)
-               : "memory");
-}
 __device__ __forceinline__ void cp_async16_s(uint32_t dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
@@ -237,9 +258,8 @@ __device__ __forceinline__ bool row_wait_count(const int* p, int target, int* cn
   }
 }
 
-template <int NM_, int NT, bool BATCH, class PP>
+template <class C, bool BATCH, class PP>
 __device__ __forceinline__ void row_tasker(const PP& P, int cls, double* smem) {
-  using C = RowCfg<NM_, NT>;
   const int lane = threadIdx.x & 31;
   int* const cnt = reinterpret_cast<int*>(smem + C::SM_CNT);
   int* const sync = P.sy.sync;
@@ -325,24 +345,9 @@ __device__ __forceinline__ void row_tasker(const PP& P, int cls, double* smem) {
     } else {
       Q = P.pr;
     }
-    // matrices in fragment order, zero beyond the last angle: 8-byte
-    // asynchronous copies, all in flight while the dependencies are waited for
-    double* const mat = mats + (k & 1) * C::MAT;
-    const size_t as = Q.a_stride ? (size_t)Q.a_stride : (size_t)Q.na;
-#pragma unroll 4
-    for (int e = lane; e < C::KS * NT * 32; e += 32) {
-      const int tt = (e >> 5) % NT, ks = (e >> 5) / NT;
-      const int ia = 8 * tt + (lane >> 2), im = C::KS * (lane & 3) + ks;
-      const bool in = ia < Q.na;
-      cp_async8_zfill(&mat[e], &Q.afm[in ? ia + as * (im + (size_t)NM_ * oct) : 0], in);
-    }
-#pragma unroll 4
-    for (int e = lane; e < C::MT * NT * 2 * 32; e += 32) {
-      const int i = (e >> 5) & 1, tt = (e >> 6) % NT, mt = (e >> 6) / NT;
-      const int ia = 8 * tt + 2 * (lane & 3) + i, im = 8 * mt + (lane >> 2);
-      const bool in = ia < Q.na && im < NM_;
-      cp_async8_zfill(&mat[C::KS * NT * 32 + e], &Q.mfa[in ? im + (size_t)NM_ * (ia + as * oct) : 0], in);
-    }
+    // the octant's matrices; their copies are in flight while the
+    // dependencies are waited for
+    C::load_matrices(mats + (k & 1) * C::MAT, Q, oct, lane);
     cp_async_commit();
     const int depx = (mode & DM_X_PLANE) ? r[TK_DEP_X] : -1;
     const int depy = (mode & DM_Y_PLANE) ? r[TK_DEP_Y] : -1;
@@ -377,9 +382,8 @@ __device__ __forceinline__ void row_tasker(const PP& P, int cls, double* smem) {
   }
 }
 
-template <int NM_, int NT, bool BATCH, class PP>
+template <class C, bool BATCH, class PP>
 __device__ __forceinline__ void row_fetcher(const PP& P, double* smem) {
-  using C = RowCfg<NM_, NT>;
   constexpr int E = C::E, DY = C::DY, R = C::R;
   const int lane = threadIdx.x & 31;
   int* const cnt = reinterpret_cast<int*>(smem + C::SM_CNT);
@@ -511,9 +515,8 @@ __device__ __forceinline__ void row_fetcher(const PP& P, double* smem) {
   __syncwarp();
 }
 
-template <int NM_, int NT, bool BATCH, class PP>
+template <class C, bool BATCH, class PP>
 __device__ __forceinline__ void row_publisher(const PP& P, double* smem) {
-  using C = RowCfg<NM_, NT>;
   const int lane = threadIdx.x & 31;
   int* const cnt = reinterpret_cast<int*>(smem + C::SM_CNT);
   int* const progress = P.sy.sync + SY_PROGRESS;
@@ -883,9 +886,8 @@ __device__ __forceinline__ void row_compute(const PP& P, double* smem) {
 
 // Barriers and counters of one body: set up before its first task, and
 // invalidated before another body reuses the memory.
-template <int NM_, int NT>
+template <class C>
 __device__ __forceinline__ void row_setup(double* smem, bool init) {
-  using C = RowCfg<NM_, NT>;
   uint64_t* const bars = reinterpret_cast<uint64_t*>(smem + C::SM_BAR);
   if (init) {
     for (int i = 0; i < C::NBAR; ++i) mbar_init(&bars[i], 1);
@@ -898,25 +900,24 @@ __device__ __forceinline__ void row_setup(double* smem, bool init) {
 }
 
 // The producer warps of one body.
-template <int NM_, int NT, bool BATCH, class PP>
+template <class C, bool BATCH, class PP>
 __device__ __forceinline__ void row_producers(const PP& P, int cls, double* smem) {
-  using C = RowCfg<NM_, NT>;
   const int warp = threadIdx.x >> 5;
-  if (warp == C::R) row_tasker<NM_, NT, BATCH>(P, cls, smem);
-  else if (warp == C::R + 1) row_fetcher<NM_, NT, BATCH>(P, smem);
-  else if (warp == C::R + 2) row_publisher<NM_, NT, BATCH>(P, smem);
+  if (warp == C::R) row_tasker<C, BATCH>(P, cls, smem);
+  else if (warp == C::R + 1) row_fetcher<C, BATCH>(P, smem);
+  else if (warp == C::R + 2) row_publisher<C, BATCH>(P, smem);
 }
 
 template <int NM_, int NT>
 __global__ void __launch_bounds__(RowCfg<NM_, NT>::NTH, 1) sweep_fp64_row_kernel(const Fp64Params P) {
   using C = RowCfg<NM_, NT>;
   extern __shared__ __align__(128) double smem[];
-  if (threadIdx.x == 0) row_setup<NM_, NT>(smem, true);
+  if (threadIdx.x == 0) row_setup<C>(smem, true);
   __syncthreads();
   // 384 threads x 168 registers: 8 warps x 32 x 208 + 4 x 32 x 80
   if ((threadIdx.x >> 5) >= C::R) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(80));
-    row_producers<NM_, NT, false>(P, 0, smem);
+    row_producers<C, false>(P, 0, smem);
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(208));
     row_compute<NM_, NT, false>(P, smem);

@@ -4,8 +4,6 @@
 // flags as the reference, then builds the task schedule and the device
 // buffers (face planes per octant, schedule, progress counters).
 // Sweeper_sweep (sweeper_kba_c.h:588-845) is one persistent kernel launch.
-#include <cuda.h>
-#include <cudaTypedefs.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -20,20 +18,19 @@
 #include "sweep_fp64_chain.cuh"
 #include "sweep_fp64_row.cuh"
 #include "sweep_fp64_ws.cuh"
-#include "sweep_mixed_tc.cuh"
+#include "sweep_mixed_row.cuh"
 
 namespace msb {
 
 namespace {
 
 using KernelFn = void (*)(const Fp64Params);
-using MixKernelFn = void (*)(const MixParams);
 using MixConvFn = void (*)(const double*, unsigned char*, int, int, int, int, int, int, int);
 
-// One compiled kernel: the FP64 kernel (fn) or a mixed-precision one (mix).
+// One compiled kernel: an FP64 one or the mixed-precision one (mix).
 struct Variant {
   KernelFn fn = nullptr;
-  MixKernelFn mix = nullptr;
+  bool mix = false;
   MixConvFn conv = nullptr;  // mixed precision: vi into the first transform's operand format
   size_t smem = 0;
   size_t entry_bytes = 0;  // one face entry (octant, group pair, position)
@@ -45,8 +42,10 @@ struct Variant {
   size_t row_smem[4] = {0, 0, 0, 0};
   int rw = 0;
   int gpt() const { return rw ? 8 / rw : 1; }  // group pairs per task
-  bool valid() const { return fn || mix; }
-  const void* func() const { return fn ? (const void*)fn : (const void*)mix; }
+  bool valid() const { return fn != nullptr; }
+  const void* func() const { return (const void*)fn; }
+  // body of the row kernels for a pass of nac angles
+  int body(int nac) const { return mix ? (nac > 16 ? 3 : 1) : (nac + 7) / 8 - 1; }
 };
 
 constexpr int kStages = 4;
@@ -139,31 +138,37 @@ Variant pick_nch(int nch, int tile) {
   }
 }
 
-constexpr int kMixStages = 4;
-
+// The mixed-precision row kernel (bodies for passes of 16 and 32 angles).
 template <int NM_, int FMT>
-Variant make_mixed() {
-  using C = MixCfg<NM_, kMixStages>;
-  static_assert(C::smem_bytes() + 128 <= 227 * 1024, "shared memory budget (dynamic + static)");
+Variant make_mixed(int rw, int na) {
+  static_assert(MixRowCfg<NM_, FMT, 4>::smem_bytes() <= 227 * 1024, "shared memory budget");
   Variant v;
-  v.mix = sweep_mixed_kernel<NM_, FMT, kMixStages>;
+  v.mix = true;
+  v.row_fn[1] = sweep_mixed_row_kernel<NM_, FMT, 2>;
+  v.row_fn[3] = sweep_mixed_row_kernel<NM_, FMT, 4>;
+  v.row_smem[1] = MixRowCfg<NM_, FMT, 2>::smem_bytes();
+  v.row_smem[3] = MixRowCfg<NM_, FMT, 4>::smem_bytes();
   v.conv = convert_vi16<NM_, FMT>;
-  v.smem = C::smem_bytes();
-  v.entry_bytes = C::EB;
-  v.tx = C::TX;
-  v.ty = C::TY;
+  const int b = v.body(std::min(na, 32));  // of the widest pass
+  v.fn = v.row_fn[b];
+  v.smem = v.row_smem[b];
+  v.entry_bytes = (size_t)(b + 1) * 64 * sizeof(float);
+  v.tx = 4;
+  v.ty = rw;
   v.nch = 1;
-  v.threads = C::NT;
+  v.threads = 384;
   v.pass = 32;
+  v.kernel = 2;
+  v.rw = rw;
   return v;
 }
 
 template <int FMT>
-Variant pick_mixed(int nm) {
+Variant pick_mixed(int nm, int rw, int na) {
   switch (nm) {
-    case 4: return make_mixed<4, FMT>();
-    case 8: return make_mixed<8, FMT>();
-    case 16: return make_mixed<16, FMT>();
+    case 4: return make_mixed<4, FMT>(rw, na);
+    case 8: return make_mixed<8, FMT>(rw, na);
+    case 16: return make_mixed<16, FMT>(rw, na);
     default: return Variant();
   }
 }
@@ -180,11 +185,11 @@ Variant pick_chain(int tile) {
 // angles per pass (the transform matrices stay in registers), 64 = two
 // 32-angle chunks per pass (matrices read from shared memory; slower per
 // angle).  na <= 128; the mixed kernels sweep 32 angles per pass.
-Variant pick_variant(int nm, int na, int precision, int tile = 0, int kernel = 0, int angle_pass = 0) {
+Variant pick_variant(int nm, int na, int precision, int tile = 0, int kernel = 0, int angle_pass = 0, int rw = 8) {
   if (na > 128) return Variant();
   if (precision == 1 || precision == 2) {
     if (tile != 0) return Variant();
-    return precision == 1 ? pick_mixed<MIX_F16>(nm) : pick_mixed<MIX_BF16>(nm);
+    return precision == 1 ? pick_mixed<MIX_F16>(nm, rw, na) : pick_mixed<MIX_BF16>(nm, rw, na);
   }
   if (precision != 0) return Variant();
   if (kernel == 1) {
@@ -342,7 +347,7 @@ static int setup_plan(const SweeperImpl& S, const Variant& var, int window, Sche
     return rc;
   const int rem = dims.na % 32;  // the row kernel's body for a last pass of fewer angles
   if (var.rw && rem) {
-    const int b = (rem + 7) / 8 - 1;
+    const int b = var.body(rem);
     if ((rc = cuda_check(cudaFuncSetAttribute((const void*)var.row_fn[b], cudaFuncAttributeMaxDynamicSharedMemorySize,
                                               (int)var.row_smem[b]),
                          "cudaFuncSetAttribute")))
@@ -376,6 +381,8 @@ static int impl_create(SweeperImpl& S, const Dimensions& dims, int precision, in
   if ((rc = cuda_check(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev), "SM count"))) return rc;
   S.nsm = nsm;
   // no flag asks for a shape or a kernel: the row kernel
+  if (S.var.mix)
+    S.var = pick_variant(dims.nm, dims.na, precision, 0, 0, 0, pick_rows(dims.ncell_x, dims.ncell_y, S.ngp, 4 * nsm));
   if (precision == 0 && kernel == 0 && tile == 0 && angle_pass == 0 && !autotune)
     S.var = pick_row(dims.nm, dims.na, pick_rows(dims.ncell_x, dims.ncell_y, S.ngp, 4 * nsm));
   if ((rc = setup_plan(S, S.var, S.window, S.sched, S.gp_block, S.d_tasks, S.grid))) return rc;
@@ -484,16 +491,15 @@ static int reset_pass(SweeperImpl& S, cudaStream_t stream) {
                     "reset sync");
 }
 
-// Problem fields (X) and schedule fields (P) of a launch; F is the face type.
-template <class F, class X, class PP>
-static void fill_params(const SweeperImpl& S, X& x, PP& P, const double* vi_d, const int* d_tasks, long long ntask) {
-  if constexpr (std::is_same<X, Fp64Prob>::value) x.vi = vi_d;  // the mixed sweep reads vi16 instead
-  else (void)vi_d;
+// Problem and schedule fields of a launch.
+static void fill_params(const SweeperImpl& S, Fp64Params& P, const double* vi_d, const int* d_tasks, long long ntask) {
+  Fp64Prob& x = P.pr;
+  x.vi = vi_d;
   x.afm = S.d_afm;
   x.mfa = S.d_mfa;
-  x.fxy = static_cast<F*>(S.d_face[0]);
-  x.fxz = static_cast<F*>(S.d_face[1]);
-  x.fyz = static_cast<F*>(S.d_face[2]);
+  x.fxy = static_cast<double*>(S.d_face[0]);
+  x.fxz = static_cast<double*>(S.d_face[1]);
+  x.fyz = static_cast<double*>(S.d_face[2]);
   x.nx = S.dims.ncell_x;
   x.ny = S.dims.ncell_y;
   x.nz = S.dims.ncell_z;
@@ -502,10 +508,9 @@ static void fill_params(const SweeperImpl& S, X& x, PP& P, const double* vi_d, c
   x.ngp = S.ngp;
   x.ia_base = 0;
   x.ie_base = S.ie_base;
-  if constexpr (std::is_same<X, Fp64Prob>::value) {
-    x.l2_hints = S.l2_hints;
-    x.sp_off = S.sp_off;
-  }
+  x.l2_hints = S.l2_hints;
+  x.sp_off = S.sp_off;
+  x.rw = (signed char)S.var.rw;
   P.tasks = d_tasks;
   P.ntask = ntask;
   P.sy.sync = S.d_sync;
@@ -519,7 +524,7 @@ static int launch_fp64(SweeperImpl& S, const Variant& var, const int* d_tasks, l
   int rc;
   for (int c = 0; c < npass; ++c) {
     Fp64Params P{};
-    fill_params<double>(S, P.pr, P, vi_d, d_tasks, ntask);
+    fill_params(S, P, vi_d, d_tasks, ntask);
     P.pr.vo = vo_d;
     P.pr.vo_add = c > 0 ? 1 : 0;  // later passes add to vo in every phase
     const int a0 = pa * c, nac = std::min(pa, na - a0);
@@ -538,8 +543,7 @@ static int launch_fp64(SweeperImpl& S, const Variant& var, const int* d_tasks, l
       }
     }
     if (var.rw) {
-      const int b = (nac + 7) / 8 - 1;
-      P.pr.rw = (signed char)var.rw;
+      const int b = var.body(nac);
       var.row_fn[b]<<<grid, var.threads, var.row_smem[b], stream>>>(P);
     } else {
       var.fn<<<grid, var.threads, var.smem, stream>>>(P);
@@ -557,31 +561,31 @@ static int launch_mixed(SweeperImpl& S, double* vo_d, const double* vi_d, cudaSt
                         const int* d_tasks, long long ntask, int gp0, int gp1) {
   const int na = S.dims.na, pa = pass_angles(S), npass = (na + pa - 1) / pa;
   const Dimensions& d = S.dims;
-  MixParams P;
-  fill_params<float>(S, P, P, vi_d, d_tasks, ntask);
-  P.part = S.d_part;
-  P.state = S.part_elems / NOCTANT;
+  // the kernel's vi is the converted one, its vo the octants' FP32 partials
+  Fp64Params P{};
+  fill_params(S, P, reinterpret_cast<const double*>(S.d_vi16), d_tasks, ntask);
+  P.pr.vo = reinterpret_cast<double*>(S.d_part);
+  const size_t state = S.part_elems / NOCTANT;
   int rc;
   // vi in the first transform's operand format, once for every octant and pass
   S.var.conv<<<S.nsm * 8, 256, 0, stream>>>(vi_d, S.d_vi16, d.ncell_x, d.ncell_y, d.ncell_z, d.ne, S.ngp, gp0,
                                             gp1);
   if ((rc = cuda_check(cudaGetLastError(), "vi conversion launch"))) return rc;
-  P.vi16 = S.d_vi16;
   for (int c = 0; c < npass; ++c) {
-    if (npass > 1) {
-      const int a0 = pa * c, nac = std::min(pa, na - a0);
-      if ((rc = copy_pass_matrices(S, a0, nac, stream))) return rc;
+    const int a0 = pa * c, nac = std::min(pa, na - a0), b = S.var.body(nac);
+    if (npass > 1) {  // the pass's angles read in place
       if (c > 0 && (rc = reset_pass(S, stream))) return rc;
-      P.afm = S.d_afm_c;
-      P.mfa = S.d_mfa_c;
-      P.na = nac;
-      P.ia_base = a0;
+      P.pr.afm = S.d_afm + a0;
+      P.pr.mfa = S.d_mfa + (size_t)a0 * d.nm;
+      P.pr.a_stride = na;
+      P.pr.na = nac;
+      P.pr.ia_base = a0;
     }
-    S.var.mix<<<S.grid, S.var.threads, S.var.smem, stream>>>(P);
+    S.var.row_fn[b]<<<S.grid, S.var.threads, S.var.row_smem[b], stream>>>(P);
     if ((rc = cuda_check(cudaGetLastError(), "sweep kernel launch"))) return rc;
     const size_t layer = (size_t)d.nm * NU * d.ncell_x * d.ncell_y;  // one (iz, ie) slab
     const int e0 = 2 * gp0, e1 = std::min(2 * gp1, d.ne);
-    reduce_octant_partials<<<S.nsm * 8, 256, 0, stream>>>(vo_d, S.d_part, P.state, c > 0 ? 1 : 0, layer * d.ne,
+    reduce_octant_partials<<<S.nsm * 8, 256, 0, stream>>>(vo_d, S.d_part, state, c > 0 ? 1 : 0, layer * d.ne,
                                                           layer * e0, layer * (e1 - e0), d.ncell_z);
     if ((rc = cuda_check(cudaGetLastError(), "partial sum launch"))) return rc;
   }
@@ -632,7 +636,7 @@ static int impl_sweep(SweeperImpl& S, double* vo_d, const double* vi_d, const do
   int rc;
   if ((rc = load_matrices(S, afm_h, mfa_h, afm_d, mfa_d, stream))) return rc;
   if ((rc = cuda_check(cudaMemsetAsync(S.d_sync, 0, S.sync_ints * sizeof(int), stream), "reset sync"))) return rc;
-  if (S.var.fn && S.autotune && !S.tuned) {
+  if (!S.var.mix && S.autotune && !S.tuned) {
     // First sweep of an autotuning sweeper: the same sweep with the sweeper's
     // own plan and with every candidate (each writes all of vo), timed on the
     // stream; the fastest plan is kept for every later sweep.
@@ -683,7 +687,7 @@ static int impl_sweep(SweeperImpl& S, double* vo_d, const double* vi_d, const do
     for (const auto& a : S.alts)
       if (a.var.tx != S.var.tx && (S.tune_ms[1] == 0.f || a.ms < S.tune_ms[1])) S.tune_ms[1] = a.ms;
     // the sync words hold the last trial's status, which was clean
-  } else if (S.var.fn) {
+  } else if (!S.var.mix) {
     if ((rc = launch_fp64(S, S.var, S.d_tasks, S.sched.ntask(), S.grid, vo_d, vi_d, stream))) return rc;
   } else {
     if ((rc = launch_mixed(S, vo_d, vi_d, stream, S.d_tasks, S.sched.ntask(), 0, S.ngp))) return rc;
@@ -841,7 +845,7 @@ static int sweep_iterations_sliced(SweeperImpl& S, int nslice, double* out_h, co
     for (int it = 0; it < niterations && !rc; ++it) {
       if (k > 0 || it > 0) rc = reset_pass(S, st);
       if (!rc)
-        rc = S.var.fn ? launch_fp64(S, S.var, T.d_tasks[k], T.ntask[k], S.grid, b, a, st)
+        rc = !S.var.mix ? launch_fp64(S, S.var, T.d_tasks[k], T.ntask[k], S.grid, b, a, st)
                       : launch_mixed(S, b, a, st, T.d_tasks[k], T.ntask[k], T.gp0[k], T.gp0[k + 1]);
       std::swap(a, b);
     }
@@ -1030,7 +1034,7 @@ static int kba_step(SweeperImpl& S, int step, cudaStream_t stream) {
                       "reset sync");
     if (rc) break;
     Fp64Params P{};
-    fill_params<double>(S, P.pr, P, K.vi_d, K.d_tasks + K.off[k] * MSB_TASK_INTS, K.cnt[k]);
+    fill_params(S, P, K.vi_d, K.d_tasks + K.off[k] * MSB_TASK_INTS, K.cnt[k]);
     P.pr.vo = K.vo_d;
     P.pr.vo_add = c > 0 ? 1 : 0;
     P.pr.fxy = reinterpret_cast<double*>(static_cast<char*>(S.d_face[0]) + c * K.plane_pass[0]);
