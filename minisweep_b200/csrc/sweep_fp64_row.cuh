@@ -589,39 +589,57 @@ __device__ __forceinline__ void row_compute(const PP& P, double* smem) {
   for (int i = 0; i < 2; ++i) wz[i] = 1.0 / 4.0 - 1.0 / (double)(1 << (2 * r + i));
 
   uint32_t x_ph = 0;                              // phase of the entering x face
-  bool handed = false;           // the fetcher filled the next warp's ring since this warp last did
-  uint32_t n_in = 0, n_out = 0;  // y faces that passed through this warp's ring and the next warp's, earlier tasks
+  // y rings, this warp's (in) and the next warp's (out): positions and phases
+  // (an empty slot's phase lags by one)
+  uint32_t yi = 0, yi_ph = 0, yo = 0, yo_ph = 1;
+  // A batch changes the pipeline height from task to task, and with it who
+  // fills a ring: it counts the faces that passed through each in earlier tasks.
+  bool handed = false;  // the fetcher filled the next warp's ring since this warp last did
+  uint32_t n_in = 0, n_out = 0;
+  int rw = 8, row = 0, pipe = 0;
+  if constexpr (!BATCH) {
+    rw = P.pr.rw;
+    row = warp % rw;
+    pipe = warp / rw;
+  }
   for (int k = 0;; ++k) {
     if (!row_wait_count(cnt + RC_POSTED, k + 1, cnt, P.sy, 64)) return;
     const RowRec& rec = reinterpret_cast<const RowRec*>(smem + C::SM_REC)[k % C::NREC];
     if (rec.stop) return;
-    const int oct = rec.oct, flags = rec.flags;
-    int rw;
-    if constexpr (BATCH) rw = rec.rw; else rw = P.pr.rw;
-    const int row = warp % rw, gp = rec.gp * (R / rw) + warp / rw;
+    if constexpr (BATCH) {
+      rw = rec.rw;
+      row = warp % rw;
+      pipe = warp / rw;
+    }
+    const int oct = rec.oct, flags = rec.flags, gp = rec.gp * (R / rw) + pipe;
     const Fp64Prob& Q = rec.q;
     const int w = rec.x1 - rec.x0, h = rec.y1 - rec.y0, nzr = rec.z1 - rec.z0;
     const bool runs = row < h && gp < Q.ngp;
-    const bool y_feed = runs && (row > 0 || (flags & TF_Y_IN));  // the y face comes through the ring
-    const bool y_pass = runs && row + 1 < min(h, rw);            // ... and goes on through the next one
-    // ring positions and phases (an empty slot's phase lags by one)
-    uint32_t yi = n_in % DY, yi_ph = (n_in / DY) & 1, yo = n_out % DY, yo_ph = (n_out / DY + 1) & 1;
-    if (y_feed) n_in += w * nzr;
-    // the next warp's ring also takes faces where that warp begins a pipeline
-    // and the fetcher feeds it
-    const int row2 = (warp + 1) % rw, gp2 = rec.gp * (R / rw) + (warp + 1) / rw;
-    const bool fetched = row2 == 0 && gp2 < Q.ngp && (flags & TF_Y_IN);
-    if (y_pass || fetched) n_out += w * nzr;
-    if (y_pass && handed) {  // as in the fetcher: a ring that changes its producer
-      if (!row_wait_count(cnt + RC_PLANES + warp + 1, rec.plane0, cnt, P.sy, 64)) return;
-      handed = false;
+    if constexpr (BATCH) {
+      yi = n_in % DY;
+      yi_ph = (n_in / DY) & 1;
+      yo = n_out % DY;
+      yo_ph = (n_out / DY + 1) & 1;
+      const bool passes = runs && row + 1 < h;
+      if (runs && (row > 0 || (flags & TF_Y_IN))) n_in += w * nzr;
+      // the next warp's ring also takes faces where that warp begins a pipeline
+      // and the fetcher feeds it
+      const int gp2 = rec.gp * (R / rw) + (warp + 1) / rw;
+      const bool fetched = (warp + 1) % rw == 0 && gp2 < Q.ngp && (flags & TF_Y_IN);
+      if (passes || fetched) n_out += w * nzr;
+      if (passes && handed) {  // as in the fetcher: a ring that changes its producer
+        if (!row_wait_count(cnt + RC_PLANES + warp + 1, rec.plane0, cnt, P.sy, 64)) return;
+        handed = false;
+      }
+      if (fetched) handed = true;
     }
-    if (fetched) handed = true;
     if (!runs) {
       __syncwarp();
       if (lane == 0) st_release_cta(cnt + RC_PLANES + warp, rec.plane0 + nzr);
       continue;
     }
+    const bool y_feed = row > 0 || (flags & TF_Y_IN);  // the y face comes through the ring
+    const bool y_pass = row + 1 < h;                   // ... and goes on through the next one
     const int dx = (oct & 1) ? -1 : 1, dy = (oct & 2) ? -1 : 1, dz = (oct & 4) ? -1 : 1;
     const bool first = (flags & TF_FIRST) != 0 && !Q.vo_add;
     const int ix0 = dx > 0 ? rec.x0 : rec.x1 - 1, iz0 = dz > 0 ? rec.z0 : rec.z1 - 1;
