@@ -66,9 +66,11 @@ struct RowCfg {
   static constexpr int E = NT * 64;           // doubles per face entry (8 columns x 8 NT angles)
   static constexpr int VSZ = 2 * NM_ * NU;    // doubles of vi (or vo) per cell and group pair
   // input ring of a warp, in cells: 4 x 2 KB at 16 moments; a cell of 8 or 4
-  // moments takes less time and less room, so 8
-  static constexpr int D = NM_ == 16 ? 4 : 8;
-  static constexpr int DY = 3;                // y faces between two rows
+  // moments takes less time and less room
+  static constexpr int D = NM_ == 16 ? 4 : NM_ == 8 ? 6 : 8;
+  // y faces between two rows: as many as fit, since the rows do not run
+  // evenly (37 x 29 x 41, ne 23, na 45, nm 8: 6.53 ms with 3, 6.23 so)
+  static constexpr int DY = NT <= 2 ? 6 : NT == 3 ? 5 : NM_ == 16 ? 3 : NM_ == 8 ? 4 : 5;
   static constexpr int NREC = 4;              // task records
   static constexpr int MAT = (KS + MT * 2) * NT * 32;
   static constexpr int SM_ZC = 0;                       // [R][W][E]
