@@ -129,7 +129,7 @@ def measured_peaks() -> dict:
         return {"hbm_gbs": 6650.0, "bf16_tflops": 1590.0, "source": "fallback (earlier measurement on this pool)"}
 
 
-def profile_traffic(kernel: str = "sweep_fp64_kernel") -> float | None:
+def profile_traffic(kernel: str = "sweep_fp64_row_kernel") -> float | None:
     """DRAM bytes per 64^3 sweep of a kernel from its committed ncu summary."""
     try:
         with open(os.path.join(ROOT, "profiles", kernel + ".md")) as f:
@@ -331,9 +331,9 @@ def measure_mixed(args, pb64, flags, va, vb, stream, dev, world, ms_fp64=None) -
                     "roofline": {"bound": "hbm", "achieved": hbm, "peak": peaks.get("hbm_gbs"), "unit": "GB/s",
                                  "peak_source": peaks.get("source"),
                                  "frac": hbm / peaks["hbm_gbs"] if peaks.get("hbm_gbs") else None,
-                                 "traffic": profile_traffic("sweep_mixed_kernel"),
-                                 "traffic_source": "constant read from profiles/sweep_mixed_kernel.md: ncu DRAM "
-                                                   "bytes of one 32^3 x ne 32 sweep scaled x16; not measured in "
+                                 "traffic": profile_traffic("sweep_mixed_row_kernel"),
+                                 "traffic_source": "constant read from profiles/sweep_mixed_row_kernel.md: ncu DRAM "
+                                                   "bytes of one 32^3 x ne 16 sweep scaled x32; not measured in "
                                                    "this run",
                                  "algorithmic": "16 x state bytes per sweep (vi read + vo write) / mean sweep "
                                                 "kernel time"}})
@@ -741,8 +741,8 @@ def run_ours(args, rank: int, world: int, local_rank: int) -> int:
         roofline = {"bound": "tensor", "achieved": tf, "peak": peak_dmma, "unit": "TFLOP/s",
                     "frac": tf / peak_dmma if peak_dmma else None,
                     "traffic": traffic,
-                    "traffic_source": "constant read from profiles/sweep_fp64_kernel.md: ncu DRAM bytes of one "
-                                      "32^3 x ne 32 sweep scaled x16 to this workload; not measured in this run",
+                    "traffic_source": "constant read from profiles/sweep_fp64_row_kernel.md: ncu DRAM bytes of one "
+                                      "32^3 x ne 16 sweep scaled x32 to this workload; not measured in this run",
                     "peak_source": "FP64 mma.sync peak measured live by msb_measure_fp64_peak (MEASURED_PEAKS.json "
                                    "has no FP64 figure); FMA-pipe FP64 peak %.2f TF/s" % peak_dfma,
                     "algorithmic": "reference flop model (runner.c:162-166) %.4g flop per sweep / mean sweep "
@@ -775,7 +775,7 @@ def run_ours(args, rank: int, world: int, local_rank: int) -> int:
                     "tile": {"cells_per_cta": [tile["tx"], tile["ty"]],
                              "autotune_first_sweep_ms": {"chosen": tile["ms_chosen"],
                                                          "best_other_tile": tile["ms_other"]}},
-                    "plan": {"fp64_kernel": "chained wavefront" if tile["fp64_kernel"] else "staged",
+                    "plan": {"fp64_kernel": ("staged", "chained wavefront", "rows")[tile["fp64_kernel"]],
                              "task_window_x_sms": tile["task_window"], "l2_hints": tile["l2_hints"],
                              "angles_per_pass": tile["angle_pass"], "plans_timed": tile["candidates"]},
                     "roofline": roofline, "cpu_baseline": cpu,

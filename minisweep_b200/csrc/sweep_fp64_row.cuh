@@ -18,7 +18,7 @@
 // and 56 FP64 instructions of the solve (2 cycles each): 624 cycles at 16
 // moments and 32 angles, 1250 for the two warps of a scheduler; and 3 KB of
 // state and 4 KB (1/4 + 1/rw) of faces cross L2.  Measured, 64^3 cells x 64
-// groups, ms per sweep: 57.3 (rw 8; 2040 cycles per two cells, DRAM at 5.3
+// groups, ms per sweep: 57.6 (rw 8; 2040 cycles per two cells, DRAM at 4.9
 // TB/s), 63.0 (rw 2), the staged kernel 120.2.  What got it there from 92:
 // the vi / vo copies issued by the compute warps themselves (one warp feeding
 // all eight by bulk copies was the bound: 92 -> 81), then a cell body without

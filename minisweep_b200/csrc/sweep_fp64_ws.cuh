@@ -80,7 +80,7 @@ struct Fp64Params {
 
 // Many problems per launch.  Tasks of all problems share one table with
 // global task ids; the problems are grouped in classes (moment count, angle
-// chunks, tile shape), each class a contiguous range of the table that the
+// tiles), each class a contiguous range of the table that the
 // CTAs work through in class order.  A problem whose face planes reuse the
 // scratch of earlier problems waits until those have completed every task.
 constexpr int kMaxBatchClasses = 16;

@@ -33,6 +33,13 @@
 // round trip through shared-memory operands, a commit, an mbarrier and a
 // tensor-memory load per step, with all warps in lockstep, was what bounded
 // that form (3 % tensor pipe).
+//
+// What bounds it: instruction issue (55 % of the slots with two warps per
+// scheduler): about 430 warp instructions a cell, 190 of them the FP32 solve
+// with its error terms, 18 products.  Measured, ms per sweep (conversion and
+// partial sum included): 64^3 x 64 groups 66.5 (FP16) / 67.3 (BF16), the
+// CTA-wide form 91.6 / 92.8; 64^3 x 16 16.6 / 23.4.  With 12 rows and 128
+// registers 16.5: the third warp gains what 32 rows in tiles of 12 lose.
 #pragma once
 
 #include <cuda_bf16.h>
