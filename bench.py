@@ -451,10 +451,12 @@ def measure_batched(args, dev, world: int, rank: int, local_rank: int) -> dict |
             i1 = b1.info()
         singles_ms.append(i1["sim_makespan"])
         singles_busy.append(i1["sim_busy"])
+    with msb.Batch(probs, plan_nsm=info["nsm"], scratch_bytes=info["scratch_bytes"]) as ball:
+        batched_ms = ball.info()["sim_makespan"]
     sm_, sb_ = np.array(singles_ms), np.array(singles_busy)
     sim = {"busy_batched": info["sim_busy"], "busy_one_at_a_time_work_weighted": float((sm_ * sb_).sum() / sm_.sum()),
            "busy_one_at_a_time_min": float(sb_.min()),
-           "predicted_speedup_vs_unbatched": float(sm_.sum() / info["sim_makespan"]),
+           "predicted_speedup_vs_unbatched": float(sm_.sum() / batched_ms),
            "note": "host-side list-scheduling simulation of the planner (task durations from their wavefront "
                    "steps): one problem alone already keeps the SMs this busy, so a shared launch can recover "
                    "at most the difference"}
