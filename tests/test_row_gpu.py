@@ -44,3 +44,23 @@ def test_row_kernel_edges(nx, ny, nz, ne, na, nm, ty):
     assert np.array_equal(vo, staged)
     ref = oracle.sweep(nx, ny, nz, ne, nm, na, a, m, vi)
     assert np.max(np.abs(vo - ref)) <= 1e-12 * np.max(np.abs(ref))
+
+
+@pytest.mark.parametrize("prec,bound", [(1, 1e-6), (2, 2e-5)])
+@pytest.mark.parametrize("nx,ny,nz,ne,na,nm,ty", [
+    (1, 1, 1, 1, 1, 16, 8),      # one cell of a pair, the 16-angle body
+    (5, 9, 3, 3, 16, 8, 8),      # row widths 3 and 2, a row more than a pipeline
+    (8, 16, 2, 4, 17, 16, 8),    # whole tiles, the 32-angle body
+    (6, 7, 4, 2, 45, 4, 8),      # a 16-angle second pass
+    (20, 5, 4, 63, 32, 16, 4),   # 2 pipelines of 4 rows, an odd group count
+    (33, 3, 2, 61, 8, 16, 2),    # 4 pipelines of 2 rows, the last task with 3
+])
+def test_mixed_row_kernel_edges(nx, ny, nz, ne, na, nm, ty, prec, bound):
+    # bounds of the mixed sweep's error on these inputs: 22-bit operand halves
+    # (FP16) and 16-bit ones (BF16), FP32 faces and partials
+    dims = (nx, ny, nz, ne, na, nm)
+    a, m, vi = oracle.random_problem(nx, ny, nz, ne, nm, na, seed=78)
+    vo, tile = sweep(dims, f"--precision {prec}", a, m, vi)
+    assert (tile["fp64_kernel"], tile["tx"], tile["ty"]) == (2, 4, ty)
+    ref = oracle.sweep(nx, ny, nz, ne, nm, na, a, m, vi)
+    assert np.max(np.abs(vo - ref)) <= bound * np.max(np.abs(ref))
