@@ -120,6 +120,7 @@ enum RowCounter {
   RC_PLANES = 0,  // [8] planes warp w has finished, over all tasks
   RC_POSTED = 8,  // tasks posted
   RC_PUBLISHED,   // tasks published complete
+  RC_FETCHED,     // tasks the fetcher is done with
   RC_QUIT
 };
 
@@ -296,8 +297,10 @@ __device__ __forceinline__ void row_tasker(const PP& P, int cls, double* smem) {
     // early enough to wait for its dependencies and lay out its matrices,
     // late enough that a reserved task does not sit behind a whole other one.
     bool ok = k == 0 || row_wait_count(cnt + RC_PLANES, max(plane_next - 4, plane0[0]), cnt, P.sy, 250);
-    // the record and the matrix buffer were last used by tasks k - 4 and k - 2
-    ok = ok && row_wait_count(cnt + RC_PUBLISHED, k - C::NREC + 1, cnt, P.sy, 64) && rows_past(plane0[0]);
+    // the record and the matrix buffer were last used by tasks k - 4 (by the
+    // rows, the publisher and the fetcher) and k - 2
+    ok = ok && row_wait_count(cnt + RC_PUBLISHED, k - C::NREC + 1, cnt, P.sy, 64) &&
+         row_wait_count(cnt + RC_FETCHED, k - C::NREC + 1, cnt, P.sy, 64) && rows_past(plane0[0]);
     int t = -1;
     if (ok && lane == 0 && ld_relaxed(&sync[SY_ABORT]) == 0) {
       if constexpr (BATCH) {
@@ -412,6 +415,8 @@ __device__ __forceinline__ void row_fetcher(const PP& P, double* smem) {
   int plane0 = 0;
   const char* src = nullptr;
   long long fa = 0, fc = 0;  // byte strides
+  bool was_live = live;
+  int done_upto = 0, k_seen = 0;  // tasks every lane is past; this lane's task last time
   for (;;) {
     bool moved = false;
     if (live && !have && ld_acquire_cta(cnt + RC_POSTED) > k) {
@@ -493,12 +498,27 @@ __device__ __forceinline__ void row_fetcher(const PP& P, double* smem) {
         }
       }
     }
-    if (__any_sync(0xffffffffu, fail)) {
+    // one vote for what the lanes did: the loop's length is the fetcher's
+    // latency, which rows of 4 and 8 moments feel (37 x 29 x 41, nm 8: 6.23 ms
+    // with three votes and no count of tasks, 6.36 with a count every time)
+    const unsigned did = __reduce_or_sync(0xffffffffu, (moved ? 1u : 0u) | (live ? 2u : 0u) | (fail ? 4u : 0u) |
+                                                           (k != k_seen || was_live != live ? 8u : 0u));
+    k_seen = k;
+    was_live = live;
+    if (did & 8u) {
+      const int past = __reduce_min_sync(0xffffffffu, live ? k : 0x7fffffff);
+      if (lane == 0 && past != done_upto) st_release_cta(cnt + RC_FETCHED, past);
+      done_upto = past;
+    }
+    if (did & 4u) {
       if (lane == 0) st_release_cta(cnt + RC_QUIT, 1);
       break;
     }
-    if (!__any_sync(0xffffffffu, live) || ld_volatile(cnt + RC_QUIT) != 0) break;
-    if (!__any_sync(0xffffffffu, moved)) __nanosleep(100);
+    if (!(did & 2u)) break;
+    if (!(did & 1u)) {
+      if (ld_volatile(cnt + RC_QUIT) != 0) break;
+      __nanosleep(40);
+    }
     __syncwarp();
   }
   __syncwarp();
