@@ -506,6 +506,7 @@ __device__ __forceinline__ void row_fetcher(const PP& P, double* smem) {
     k_seen = k;
     was_live = live;
     if (did & 8u) {
+      __syncwarp();  // what every lane read of the records it is past, before lane 0 gives them back
       const int past = __reduce_min_sync(0xffffffffu, live ? k : 0x7fffffff);
       if (lane == 0 && past != done_upto) st_release_cta(cnt + RC_FETCHED, past);
       done_upto = past;

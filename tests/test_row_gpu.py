@@ -64,3 +64,19 @@ def test_mixed_row_kernel_edges(nx, ny, nz, ne, na, nm, ty, prec, bound):
     assert (tile["fp64_kernel"], tile["tx"], tile["ty"]) == (2, 4, ty)
     ref = oracle.sweep(nx, ny, nz, ne, nm, na, a, m, vi)
     assert np.max(np.abs(vo - ref)) <= bound * np.max(np.abs(ref))
+
+
+@pytest.mark.parametrize("nx,ny,nz,ne,na,nm", [
+    (40, 40, 6, 12, 8, 4),    # 5760 tasks, both faces entering at most tiles
+    (12, 70, 3, 60, 16, 8),   # long columns of tiles, short tasks
+])
+def test_row_kernel_reuses_its_task_records(nx, ny, nz, ne, na, nm):
+    """Tens of short tasks per CTA, whose four task records the fetcher must
+    have left before the tasker writes the next task into them."""
+    a, m, vi = oracle.random_problem(nx, ny, nz, ne, nm, na, seed=79)
+    dims = (nx, ny, nz, ne, na, nm)
+    staged, _ = sweep(dims, "--tile 42", a, m, vi)
+    with msb.Problem(f"--ncell_x {nx} --ncell_y {ny} --ncell_z {nz} --ne {ne} --na {na}", nm=nm) as pb:
+        pb.set_matrices(a, m)
+        for _ in range(5):
+            assert np.array_equal(pb.sweep_host(vi), staged)
