@@ -61,8 +61,11 @@ constexpr int batch_kind(int nm, int nt) { return (nm == 4 ? 0 : nm == 8 ? 4 : 8
 // Between two classes: every warp of the CTA is done with the previous
 // class's shared memory (a barrier that warps reach from their own role's
 // code, so the non-aligned form), thread 0 swaps the barrier sets, and nobody
-// starts the new class before that.
+// starts the new class before that.  The new class's face buffers, which bulk
+// copies fill, lie over bytes that the old class and the swap wrote with
+// ordinary stores: each writer's proxy fence precedes a barrier.
 __device__ __forceinline__ void row_batch_switch(const Fp64Batch& P, int c, double* smem) {
+  fence_proxy_async_smem();
   asm volatile("barrier.sync 0;" ::: "memory");
   if (threadIdx.x == 0) {
     for (int k = 0; k < 2; ++k) {
@@ -77,6 +80,7 @@ __device__ __forceinline__ void row_batch_switch(const Fp64Batch& P, int c, doub
         default: break;
       }
     }
+    fence_proxy_async_smem();
   }
   asm volatile("barrier.sync 0;" ::: "memory");
 }

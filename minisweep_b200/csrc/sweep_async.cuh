@@ -71,6 +71,11 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t by
       : "memory");
 }
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.global;" ::: "memory"); }
+// The same for shared memory: before a bulk copy writes where ordinary
+// stores or cp.async wrote.
+__device__ __forceinline__ void fence_proxy_async_smem() {
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+}
 
 // Non-blocking test of a phase (test_wait never suspends the warp).
 __device__ __forceinline__ bool mbar_test_wait(uint64_t* b, uint32_t parity) {

@@ -462,7 +462,11 @@ __device__ __forceinline__ void row_fetcher(const PP& P, double* smem) {
     if (live && have) {
       // A ring that changes its producer may be many phases behind F, where
       // the parity says nothing: first let the warp finish the earlier tasks.
-      if (handed && ld_acquire_cta(cnt + RC_PLANES + wrp) >= plane0) handed = false;
+      // Its faces were ordinary stores; the next ones are bulk copies.
+      if (handed && ld_acquire_cta(cnt + RC_PLANES + wrp) >= plane0) {
+        fence_proxy_async_smem();
+        handed = false;
+      }
       bool go = !handed && (F < depth || mbar_test_wait(&empty[F % depth], (uint32_t)((F / depth + 1) & 1)));
       if (go && dep >= 0 && seen < c + 1) {
         seen = ld_acquire(progress + dep);

@@ -207,3 +207,25 @@ def test_batch_mixed_pipelines():
         b.sync()
     for i, p in enumerate(W):
         assert np.array_equal(D.vo[i].cpu().numpy(), single(p, D.host_vi[i])), (i, p)
+
+
+def test_batch_every_body():
+    """All twelve bodies (nm x angle tiles) in one launch, each with faces
+    copied in over bytes that the body before used for something else, and
+    within each body problems of 8, 4 and 2 rows per pipeline."""
+    W = []
+    for nm in (4, 8, 16):
+        for na in (8, 16, 24, 32):
+            for nx, ny, nz, ne in [(18, 34, 3, 2), (11, 5, 4, 9), (9, 4, 3, 16)] * 3:
+                W.append(dict(ncell_x=nx, ncell_y=ny, ncell_z=nz, ne=ne, na=na, nm=nm))
+    D = Device(W)
+    with msb.Batch(D.descs) as b:
+        for _ in range(3):
+            b.sweep(0)
+        b.sync()
+    refs = {}
+    for i, p in enumerate(W):
+        key = tuple(sorted(p.items()))
+        if key not in refs:
+            refs[key] = single(p, D.host_vi[i])
+        assert np.array_equal(D.vo[i].cpu().numpy(), refs[key]), (i, p)
