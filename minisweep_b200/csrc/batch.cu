@@ -613,8 +613,8 @@ void make_classes(BatchImpl& B) {
     ClassInfo& c = B.classes[p.cls];
     c.nm = p.d.nm;
     c.nch = p.nch;
-    c.tx = p.tx;
-    c.ty = p.rw ? 2 : p.ty;  // row kernel: its smallest pipeline
+    c.tx = p.rw ? 4 : p.tx;
+    c.ty = p.rw ? 2 : p.ty;  // row kernel: its smallest pipeline, of whole rows
   }
 }
 
@@ -625,17 +625,25 @@ int plan_batch(BatchImpl& B, const msb_problem* probs, int n, const Shape& shape
   B.probs.clear();
   B.nuser = n;
   std::vector<int> first_entry(n);
+  auto updates = [&](int i) {
+    const msb_problem& p = probs[i];
+    return (double)p.ncell_x * p.ncell_y * p.ncell_z * p.ne * p.na;
+  };
+  double all = 0.0;
+  for (int i = 0; i < n; ++i) all += updates(i);
   for (int i = 0; i < n; ++i) {
     const int npass = (probs[i].na + 31) / 32;
     first_entry[i] = (int)B.probs.size();
     auto it = shape.tile24.find(probs[i].nm);
     const bool t24 = it != shape.tile24.end() && it->second;
-    int rw = 0;
+    RowShape rs = {0, t24 ? 2 : 4};
     if (shape.device) {
       auto ir = shape.rows.find(probs[i].nm);
-      rw = ir != shape.rows.end() ? ir->second : 0;
-      // other problems fill the CTAs: no least number of tasks
-      if (!rw) rw = pick_rows(probs[i].ncell_x, probs[i].ncell_y, (probs[i].ne + 1) / 2, 0);
+      if (ir != shape.rows.end() && ir->second)
+        rs = {ir->second, 4};
+      else  // the problem's share of the SMs; other problems fill the CTAs: no least number of tasks
+        rs = pick_rows(probs[i].ncell_x, probs[i].ncell_y, probs[i].ncell_z, (probs[i].ne + 1) / 2,
+                       (int)(B.nsm * updates(i) / all), 0);
     }
     for (int c = 0; c < npass; ++c) {
       ProbPlan e;
@@ -647,10 +655,10 @@ int plan_batch(BatchImpl& B, const msb_problem* probs, int n, const Shape& shape
       e.nac = std::min(32, probs[i].na - 32 * c);
       e.prev = c > 0 ? (int)B.probs.size() - 1 : -1;
       e.nch = 1;
-      e.rw = rw;
+      e.rw = rs.rw;
       e.nt = shape.device ? std::min(4, (probs[i].na + 7) / 8) : 4;
-      e.tx = t24 ? 2 : 4;
-      e.ty = rw ? rw : t24 ? 4 : 2;
+      e.tx = rs.tx;
+      e.ty = rs.rw ? rs.rw : t24 ? 4 : 2;
       if (c > 0) B.probs.back().next = (int)B.probs.size();
       B.probs.push_back(e);
     }

@@ -78,9 +78,17 @@ int build_schedule(int nx, int ny, int nz, int ngp, int tx, int ty, int gp_block
 // about `window` tasks.
 int pick_gp_block(int nx, int ny, int ngp, int tx, int ty, int window);
 
-// Rows per pipeline of the row kernel (8, 4 or 2; a task then covers 1, 2 or 4
-// group pairs).  Fewer than 8 only with at least min_tasks tasks in a phase.
-int pick_rows(int nx, int ny, int ngp, int min_tasks);
+// How the row kernel cuts a problem: rows per pipeline (8, 4 or 2; a task then
+// covers 1, 2 or 4 group pairs) and cells per row (4, or 2 or 1 where a row of
+// 4 would be a region's whole width).
+struct RowShape {
+  int rw, tx;
+};
+
+// The shape for a problem that has `slots` SMs to itself.  Regions of more
+// than 4 rows get fewer than 8 rows a pipeline only if a cut into 8 would
+// give min_tasks tasks to a phase.
+RowShape pick_rows(int nx, int ny, int nz, int ngp, int slots, int min_tasks);
 
 // ------------------------------------------------------- KBA decomposition
 // One slab of a decomposed sweep: one octant over the process's whole x-y

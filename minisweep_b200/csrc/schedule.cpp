@@ -263,6 +263,50 @@ int pick_gp_block(int nx, int ny, int ngp, int tx, int ty, int window) {
   return b;
 }
 
+namespace {
+
+// Regions of at most 4 rows.  A task is then one chain of cells after
+// another on few warps, and how long the chain is matters as soon as a
+// phase's tasks find an SM each: group pairs share a CTA (fewer rows a
+// pipeline) only when they have to, and a row is cut in tiles of 2 or 1
+// cells, which follow each other plane by plane, where there are SMs for the
+// tiles.  A tile's plane takes 0.75 us a cell, but 1.2 at least; a tile more
+// in a row costs about 6 cells.  More pipelines in a CTA: a few per cent with
+// 2, 10 to 30 with 4 (their rows share the schedulers then).  A row is cut
+// only where one tile of 4 cells is all of it: with two tiles or more the
+// octants' phases overlap instead.
+// Measured, us per sweep, nm 16, na 32 (staged kernel; 8 rows x 4 cells; the
+// shape chosen):
+//   8 x 2 x 64, ne 2    496   801  475 (8 x 1)   ne 64   824  1375  667 (2 x 2)
+//   8 x 4 x 64, ne 16   616   837  572 (8 x 2)   ne 128 1919  2794 1129 (2 x 4)
+//   16 x 2 x 64, ne 64 1583  2744 1048 (2 x 4)
+// The staged kernel stays ahead at 9 to 18 group pairs, nm 16 and 5 to 8 cells
+// along x, by 9 % at most (8 x 2 x 96, ne 32: 735 us, 801 with the 2 x 4 chosen).
+bool pick_thin(int nx, int ny, int nz, int ngp, int slots, RowShape* out) {
+  const int hx = (nx + 1) / 2, h0 = (ny + 1) / 2, hz = (nz + 1) / 2;
+  double best = 0.0;
+  for (int tx : {4, 2, 1}) {
+    if (tx < 4 && (hx > 4 || tx >= hx)) continue;
+    for (int rw : {8, 4, 2}) {
+      if (rw < 8 && (h0 > 2 || tx == 1)) break;
+      const long long tasks = (long long)(ceil_div(hx, tx) + ceil_div(nx / 2, tx)) *
+                              (ceil_div(h0, rw) + ceil_div(ny / 2, rw)) * (nz > 1 ? 2 : 1) * ceil_div(ngp, 8 / rw);
+      if (tasks > slots) continue;
+      const double chain = hz * std::max<double>(std::min(tx, hx), 1.5) + 6.0 * (ceil_div(hx, tx) - 1);
+      // a pipeline of 3 or 4 rows: only for a clear gain
+      const double v = chain * (rw == 8 ? 1.0 : rw == 4 ? 1.05 : 1.2) * (tx < 4 && h0 > 2 ? 1.2 : 1.0);
+      if (best == 0.0 || v < best) {
+        best = v;
+        *out = {rw, tx};
+      }
+      break;
+    }
+  }
+  return best > 0.0;
+}
+
+}  // namespace
+
 // 8 rows in one pipeline move the fewest y faces and leave the most CTAs to a
 // phase; where a region's rows leave many of the 8 warps idle and there are
 // tasks enough all the same, shorter pipelines share the CTA between group
@@ -270,15 +314,17 @@ int pick_gp_block(int nx, int ny, int ngp, int tx, int ty, int window) {
 //   64 x 64 x 64, ne 64   57.3  60    63.0     48 x 20 x 48, ne 32   7.29  6.43  6.45
 //   24 x 24 x 24, ne 8    0.78  0.85  0.97     40 x 6 x 40, ne 64    4.30  2.99  3.13
 //   10 x 10 x 10, ne 30   0.31  0.36  0.36     20 x 4 x 6, ne 64     0.42  0.35  0.33
-int pick_rows(int nx, int ny, int ngp, int min_tasks) {
+RowShape pick_rows(int nx, int ny, int nz, int ngp, int slots, int min_tasks) {
   const int hx = (nx + 1) / 2, h0 = (ny + 1) / 2, h1 = ny / 2;
-  if (8LL * ceil_div(hx, 4) * ceil_div(h0, 8) * ngp < min_tasks) return 8;
+  RowShape thin;
+  if (h0 <= 4 && pick_thin(nx, ny, nz, ngp, slots, &thin)) return thin;
+  if (8LL * ceil_div(hx, 4) * ceil_div(h0, 8) * ngp < min_tasks) return {8, 4};
   // rows x group pairs that a CTA's warps stand for, idle ones included
   auto cost = [&](int rw, double faces) {
     return (ceil_div(h0, rw) + ceil_div(h1, rw)) * rw * (double)(ceil_div(ngp, 8 / rw) * (8 / rw)) * faces;
   };
   const double c8 = cost(8, 1.0), c4 = cost(4, 1.2), c2 = cost(2, 1.65);
-  return c8 <= c4 && c8 <= c2 ? 8 : c4 <= c2 ? 4 : 2;
+  return {c8 <= c4 && c8 <= c2 ? 8 : c4 <= c2 ? 4 : 2, 4};
 }
 
 }  // namespace msb

@@ -592,12 +592,18 @@ __device__ __forceinline__ void row_publisher(const PP& P, double* smem) {
   }
 }
 
+// Which of a task's warps a compute warp of the CTA is.  A scheduler holds the
+// warps w and w + 4; numbered so, the rows in use of a task with fewer rows
+// than its pipelines have (rows 0, or 0 and 1, of each pipeline) are on
+// different schedulers as far as there are four.
+__device__ __forceinline__ int row_warp(int w) { return (0x54672310 >> (4 * w)) & 7; }
+
 // One compute warp: row `warp % rw` of pipeline `warp / rw` of each task.
 template <int NM_, int NT, bool BATCH, class PP>
 __device__ __forceinline__ void row_compute(const PP& P, double* smem) {
   using C = RowCfg<NM_, NT>;
   constexpr int E = C::E, VSZ = C::VSZ, W = C::W, D = C::D, DY = C::DY, R = C::R, KS = C::KS, MT = C::MT;
-  const int lane = threadIdx.x & 31, warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
+  const int lane = threadIdx.x & 31, warp = row_warp(__shfl_sync(0xffffffffu, threadIdx.x >> 5, 0));
   const int q = lane >> 2, r = lane & 3;
   int* const cnt = reinterpret_cast<int*>(smem + C::SM_CNT);
   // shared-memory addresses of this warp's barriers, rings and face slots

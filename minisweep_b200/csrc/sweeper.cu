@@ -88,10 +88,10 @@ Variant make_chain_variant() {
   return v;
 }
 
-// The row kernel (sweep_fp64_row.cuh): rw rows of 4 cells per pipeline,
+// The row kernel (sweep_fp64_row.cuh): rw rows of tx <= 4 cells per pipeline,
 // 8 / rw pipelines (group pairs) per CTA.
 template <int NM_>
-Variant make_row_variant(int rw, int na) {
+Variant make_row_variant(RowShape shape, int na) {
   Variant v;
   v.row_fn[0] = sweep_fp64_row_kernel<NM_, 1>;
   v.row_fn[1] = sweep_fp64_row_kernel<NM_, 2>;
@@ -106,21 +106,21 @@ Variant make_row_variant(int rw, int na) {
   v.fn = v.row_fn[nt - 1];
   v.smem = v.row_smem[nt - 1];
   v.entry_bytes = (size_t)nt * 64 * sizeof(double);
-  v.tx = 4;
-  v.ty = rw;
+  v.tx = shape.tx;
+  v.ty = shape.rw;
   v.nch = 1;
   v.threads = RowCfg<NM_, 4>::NTH;
   v.pass = 32;
   v.kernel = 2;
-  v.rw = rw;
+  v.rw = shape.rw;
   return v;
 }
 
-Variant pick_row(int nm, int na, int rw) {
+Variant pick_row(int nm, int na, RowShape shape) {
   switch (nm) {
-    case 4: return make_row_variant<4>(rw, na);
-    case 8: return make_row_variant<8>(rw, na);
-    case 16: return make_row_variant<16>(rw, na);
+    case 4: return make_row_variant<4>(shape, na);
+    case 8: return make_row_variant<8>(shape, na);
+    case 16: return make_row_variant<16>(shape, na);
     default: return Variant();
   }
 }
@@ -140,7 +140,7 @@ Variant pick_nch(int nch, int tile) {
 
 // The mixed-precision row kernel (bodies for passes of 16 and 32 angles).
 template <int NM_, int FMT>
-Variant make_mixed(int rw, int na) {
+Variant make_mixed(RowShape shape, int na) {
   static_assert(MixRowCfg<NM_, FMT, 4>::smem_bytes() <= 227 * 1024, "shared memory budget");
   Variant v;
   v.mix = true;
@@ -153,22 +153,22 @@ Variant make_mixed(int rw, int na) {
   v.fn = v.row_fn[b];
   v.smem = v.row_smem[b];
   v.entry_bytes = (size_t)(b + 1) * 64 * sizeof(float);
-  v.tx = 4;
-  v.ty = rw;
+  v.tx = shape.tx;
+  v.ty = shape.rw;
   v.nch = 1;
   v.threads = 384;
   v.pass = 32;
   v.kernel = 2;
-  v.rw = rw;
+  v.rw = shape.rw;
   return v;
 }
 
 template <int FMT>
-Variant pick_mixed(int nm, int rw, int na) {
+Variant pick_mixed(int nm, RowShape shape, int na) {
   switch (nm) {
-    case 4: return make_mixed<4, FMT>(rw, na);
-    case 8: return make_mixed<8, FMT>(rw, na);
-    case 16: return make_mixed<16, FMT>(rw, na);
+    case 4: return make_mixed<4, FMT>(shape, na);
+    case 8: return make_mixed<8, FMT>(shape, na);
+    case 16: return make_mixed<16, FMT>(shape, na);
     default: return Variant();
   }
 }
@@ -185,11 +185,12 @@ Variant pick_chain(int tile) {
 // angles per pass (the transform matrices stay in registers), 64 = two
 // 32-angle chunks per pass (matrices read from shared memory; slower per
 // angle).  na <= 128; the mixed kernels sweep 32 angles per pass.
-Variant pick_variant(int nm, int na, int precision, int tile = 0, int kernel = 0, int angle_pass = 0, int rw = 8) {
+Variant pick_variant(int nm, int na, int precision, int tile = 0, int kernel = 0, int angle_pass = 0,
+                     RowShape shape = {8, 4}) {
   if (na > 128) return Variant();
   if (precision == 1 || precision == 2) {
     if (tile != 0) return Variant();
-    return precision == 1 ? pick_mixed<MIX_F16>(nm, rw, na) : pick_mixed<MIX_BF16>(nm, rw, na);
+    return precision == 1 ? pick_mixed<MIX_F16>(nm, shape, na) : pick_mixed<MIX_BF16>(nm, shape, na);
   }
   if (precision != 0) return Variant();
   if (kernel == 1) {
@@ -381,10 +382,10 @@ static int impl_create(SweeperImpl& S, const Dimensions& dims, int precision, in
   if ((rc = cuda_check(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev), "SM count"))) return rc;
   S.nsm = nsm;
   // no flag asks for a shape or a kernel: the row kernel
-  if (S.var.mix)
-    S.var = pick_variant(dims.nm, dims.na, precision, 0, 0, 0, pick_rows(dims.ncell_x, dims.ncell_y, S.ngp, 4 * nsm));
+  const RowShape shape = pick_rows(dims.ncell_x, dims.ncell_y, dims.ncell_z, S.ngp, nsm, 4 * nsm);
+  if (S.var.mix) S.var = pick_variant(dims.nm, dims.na, precision, 0, 0, 0, shape);
   if (precision == 0 && kernel == 0 && tile == 0 && angle_pass == 0 && !autotune)
-    S.var = pick_row(dims.nm, dims.na, pick_rows(dims.ncell_x, dims.ncell_y, S.ngp, 4 * nsm));
+    S.var = pick_row(dims.nm, dims.na, shape);
   if ((rc = setup_plan(S, S.var, S.window, S.sched, S.gp_block, S.d_tasks, S.grid))) return rc;
   long long ntask = S.sched.ntask();
   if (autotune) {
@@ -396,7 +397,7 @@ static int impl_create(SweeperImpl& S, const Dimensions& dims, int precision, in
     for (int rw : {8, 4, 2}) {
       if (rw > 2 && (dims.ncell_y + 1) / 2 <= 4) continue;
       AltPlan a;
-      a.var = pick_row(dims.nm, dims.na, rw);
+      a.var = pick_row(dims.nm, dims.na, {rw, 4});
       a.window = S.window;
       a.l2_hints = S.l2_hints;
       if ((rc = setup_plan(S, a.var, a.window, a.sched, a.gp_block, a.d_tasks, a.grid))) {

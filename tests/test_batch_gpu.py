@@ -229,3 +229,18 @@ def test_batch_every_body():
         if key not in refs:
             refs[key] = single(p, D.host_vi[i])
         assert np.array_equal(D.vo[i].cpu().numpy(), refs[key]), (i, p)
+
+
+@pytest.mark.parametrize("n", [1, 3, 40])
+def test_batch_thin_problems(n):
+    """Problems whose regions have at most 4 rows, alone in the batch (rows cut
+    in tiles of 1 or 2 cells) and among others (whole rows, several pipelines)."""
+    W = [dict(ncell_x=8 - k % 4, ncell_y=2 + k % 3, ncell_z=40, ne=6 + k % 5, na=(33, 16, 24)[k % 3], nm=(16, 4, 8)[k % 3])
+         for k in range(n)]
+    D = Device(W)
+    with msb.Batch(D.descs) as b:
+        for _ in range(2):
+            b.sweep(0)
+        b.sync()
+    for i, p in enumerate(W):
+        assert np.array_equal(D.vo[i].cpu().numpy(), single(p, D.host_vi[i])), (i, p)
