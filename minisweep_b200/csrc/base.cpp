@@ -201,7 +201,7 @@ static const msb_comm* grid_comm(const Env* env) {
 }
 
 extern "C" void Env_finalize(Env* env) {
-  msb::norms_trim();
+  msb::norms_release();
   if (env->stream_kernel_faces_) cudaStreamDestroy((cudaStream_t)env->stream_kernel_faces_);
   env->stream_kernel_faces_ = nullptr;
   msb::node_detach(env);

@@ -128,7 +128,7 @@ int kba_messages(const KbaPlan& plan, int proc, int step, std::vector<KbaMsg>& m
 
 // Gives back the memory that the device norms keep for their next call
 // (state_ops.cu); called when an Env is finalised.
-void norms_trim();
+void norms_release();
 
 // The node-local process group (node_comm.cpp): joined by Env_initialize when
 // the launcher's MSB_NPROC / MSB_PROC / MSB_GROUP are set; left by

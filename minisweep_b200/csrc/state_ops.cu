@@ -103,49 +103,50 @@ namespace {
 // device.  The default pool gives every byte back to the driver at the next
 // synchronisation, and every call ends with one: allocating and releasing cost
 // 0.4 ms a call (16^3 cells, 16 groups, nm 4: 437 us a call, 36 from this
-// pool).  This one
-// keeps what its calls in flight need, a chunk of at most kPoolKeep, until an
-// Env is finalised.  Calls from several threads or streams get buffers of
-// their own, ordered by the stream as with any stream-ordered allocation.
+// pool).  This one keeps what its calls in flight need, a chunk of at most
+// kPoolKeep, until an Env is finalised: that destroys the pools, so that none
+// outlives a cudaDeviceReset a host program may do between two Envs (calls in
+// flight keep their buffers, the next call makes a new pool).  Calls from
+// several threads or streams get buffers of their own, ordered by the stream
+// as with any stream-ordered allocation.  A call without an Env, which nothing
+// finalises, takes the default pool.
 constexpr int kMaxDevices = 64;
 constexpr unsigned long long kPoolKeep = 32ull << 20;
 std::mutex g_pool_mutex;
 cudaMemPool_t g_pool[kMaxDevices] = {};
 
-cudaError_t norms_alloc(double** buf, size_t bytes, cudaStream_t st) {
+cudaError_t norms_alloc(double** buf, size_t bytes, const Env* env, cudaStream_t st) {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
-  if (dev >= kMaxDevices) return cudaMallocAsync(buf, bytes, st);
-  cudaMemPool_t pool;
-  {
-    std::lock_guard<std::mutex> lock(g_pool_mutex);
-    if (!g_pool[dev]) {
-      cudaMemPoolProps props = {};
-      props.allocType = cudaMemAllocationTypePinned;
-      props.location.type = cudaMemLocationTypeDevice;
-      props.location.id = dev;
-      cudaMemPool_t p = nullptr;
-      if ((e = cudaMemPoolCreate(&p, &props)) != cudaSuccess) return e;
-      unsigned long long keep = kPoolKeep;
-      if ((e = cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep)) != cudaSuccess) {
-        cudaMemPoolDestroy(p);
-        return e;
-      }
-      g_pool[dev] = p;
+  if (!env || dev >= kMaxDevices) return cudaMallocAsync(buf, bytes, st);
+  std::lock_guard<std::mutex> lock(g_pool_mutex);
+  if (!g_pool[dev]) {
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    cudaMemPool_t p = nullptr;
+    if ((e = cudaMemPoolCreate(&p, &props)) != cudaSuccess) return e;
+    unsigned long long keep = kPoolKeep;
+    if ((e = cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep)) != cudaSuccess) {
+      cudaMemPoolDestroy(p);
+      return e;
     }
-    pool = g_pool[dev];
+    g_pool[dev] = p;
   }
-  return cudaMallocFromPoolAsync(buf, bytes, pool, st);
+  return cudaMallocFromPoolAsync(buf, bytes, g_pool[dev], st);
 }
 
 }  // namespace
 
-// Gives back what the norms' pools hold and no call uses.
-void norms_trim() {
+// Gives back the norms' pools, each once no call uses it any more.
+void norms_release() {
   std::lock_guard<std::mutex> lock(g_pool_mutex);
-  for (cudaMemPool_t p : g_pool)
-    if (p) cudaMemPoolTrimTo(p, 0);
+  for (cudaMemPool_t& p : g_pool) {
+    if (p) cudaMemPoolDestroy(p);
+    p = nullptr;
+  }
 }
 
 }  // namespace msb
@@ -155,7 +156,7 @@ extern "C" int msb_state_norms_device(const double* vi_d, const double* vo_d, si
   cudaStream_t st = env ? (cudaStream_t)env->stream_kernel_faces_ : nullptr;
   double* buf = nullptr;
   int rc;
-  if ((rc = msb::cuda_check(msb::norms_alloc(&buf, sizeof(double) * (2 * msb::kNormBlocks + 2), st), "norms alloc")))
+  if ((rc = msb::cuda_check(msb::norms_alloc(&buf, sizeof(double) * (2 * msb::kNormBlocks + 2), env, st), "norms alloc")))
     return rc;
   msb::norms_partial_kernel<<<msb::kNormBlocks, msb::kNormThreads, 0, st>>>(vi_d, vo_d, n, buf);
   msb::norms_final_kernel<<<1, msb::kNormThreads, 0, st>>>(buf, msb::kNormBlocks, buf + 2 * msb::kNormBlocks);
