@@ -391,13 +391,16 @@ static int impl_create(SweeperImpl& S, const Dimensions& dims, int precision, in
   if (autotune) {
     // candidates: the staged and the chained kernel (the staged one with 32-
     // and 64-angle passes when na > 32) x both tile shapes x task windows of
-    // 4, 8 and 16 x SMs, besides the sweeper's own plan; and the row kernel,
-    // with pipelines of more than 2 rows where a region has more than 4
+    // 4, 8 and 16 x SMs, besides the sweeper's own plan; and the row kernel in
+    // the shape a sweeper without flags takes and in every pipeline height (a
+    // region of few rows may want a high one all the same: 8 rows leave a
+    // group pair a CTA of its own)
     S.autotune = true;
-    for (int rw : {8, 4, 2}) {
-      if (rw > 2 && (dims.ncell_y + 1) / 2 <= 4) continue;
+    std::vector<RowShape> rows = {{8, 4}, {4, 4}, {2, 4}};
+    if (shape.tx != 4) rows.push_back(shape);
+    for (const RowShape& r : rows) {
       AltPlan a;
-      a.var = pick_row(dims.nm, dims.na, {rw, 4});
+      a.var = pick_row(dims.nm, dims.na, r);
       a.window = S.window;
       a.l2_hints = S.l2_hints;
       if ((rc = setup_plan(S, a.var, a.window, a.sched, a.gp_block, a.d_tasks, a.grid))) {

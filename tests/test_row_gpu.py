@@ -138,3 +138,37 @@ def test_thin_regions_keep_the_staged_kernels_speed(nx, ny, nz, ne, na, nm):
                 best = min(best, e0.elapsed_time(e1))
             ms.append(best)
     assert ms[0] <= 1.2 * ms[1], ms
+
+
+def sweep_ms(pb, vo, vi):
+    """The fastest of eight sweeps after one."""
+    st = torch.cuda.ExternalStream(pb.stream)
+    torch.cuda.synchronize()
+    ms = []
+    for _ in range(9):
+        e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        e0.record(st)
+        pb.sweep_device(vo.data_ptr(), vi.data_ptr())
+        e1.record(st)
+        torch.cuda.synchronize()
+        ms.append(e0.elapsed_time(e1))
+    return min(ms[1:])
+
+
+@pytest.mark.parametrize("nx,ny,nz,ne,na,nm", [
+    (40, 6, 40, 64, 32, 16),  # the rule takes 4 rows of 3
+    (8, 8, 20, 16, 32, 16),   # ... tiles of 4 rows of 4 or 2 cells, a CTA for each group pair
+    (8, 2, 64, 2, 32, 16),    # ... tiles of one cell
+    (24, 24, 24, 8, 32, 16),  # ... 8 rows
+])
+def test_autotune_times_the_shape_of_the_rule(nx, ny, nz, ne, na, nm):
+    """--autotune 1 has the plan of a sweeper without flags among its
+    candidates, and so keeps none that is slower (10 % for the timing of its
+    single trial)."""
+    ms = []
+    for extra in ("", "--autotune 1"):
+        with msb.Problem(f"--ncell_x {nx} --ncell_y {ny} --ncell_z {nz} --ne {ne} --na {na} {extra}", nm=nm) as pb:
+            vi = torch.rand(pb.nstate, dtype=torch.float64, device="cuda")
+            vo = torch.empty_like(vi)
+            ms.append(sweep_ms(pb, vo, vi))
+    assert ms[1] <= 1.1 * ms[0], ms
