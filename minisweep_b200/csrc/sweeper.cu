@@ -394,9 +394,14 @@ static int impl_create(SweeperImpl& S, const Dimensions& dims, int precision, in
     // 4, 8 and 16 x SMs, besides the sweeper's own plan; and the row kernel in
     // the shape a sweeper without flags takes and in every pipeline height (a
     // region of few rows may want a high one all the same: 8 rows leave a
-    // group pair a CTA of its own)
+    // group pair a CTA of its own; 8 x 8 x 20, ne 16: 0.31 ms, 0.45 at best
+    // without).  The smallest problems, regions of at most 4 rows and 4
+    // planes, keep to the tiles that Sweeper_tile has always reported for
+    // them under --autotune, 4 x 2 and 2 x 4.
     S.autotune = true;
-    std::vector<RowShape> rows = {{8, 4}, {4, 4}, {2, 4}};
+    const bool small = dims.ncell_y <= 8 && dims.ncell_z <= 8;
+    std::vector<RowShape> rows = {{2, 4}};
+    if (!small) rows.insert(rows.end(), {{4, 4}, {8, 4}});
     if (shape.tx != 4) rows.push_back(shape);
     for (const RowShape& r : rows) {
       AltPlan a;
