@@ -443,23 +443,24 @@ def measure_batched(args, dev, world: int, rank: int, local_rank: int) -> dict |
     b = msb.Batch(descs, autotune=True)
     create_s = time.time() - t0
     info = b.info()
-    # the planner's list-scheduling simulation (one worker per SM): SM time
-    # busy when the problems share one launch, and when each runs alone
+    # the planner's list-scheduling simulation (one worker per SM) of the row
+    # kernel's tasks: SM time busy when the problems share one launch, and when
+    # each runs alone, all in the shapes of the rule
     singles_ms, singles_busy = [], []
     for q in probs:
-        with msb.Batch([q], plan_nsm=info["nsm"]) as b1:
+        with msb.Batch([q], plan_nsm=info["nsm"], plan_rows=0) as b1:
             i1 = b1.info()
         singles_ms.append(i1["sim_makespan"])
         singles_busy.append(i1["sim_busy"])
-    with msb.Batch(probs, plan_nsm=info["nsm"], scratch_bytes=info["scratch_bytes"]) as ball:
-        batched_ms = ball.info()["sim_makespan"]
+    with msb.Batch(probs, plan_nsm=info["nsm"], scratch_bytes=info["scratch_bytes"], plan_rows=0) as ball:
+        batched_ms, batched_busy = ball.info()["sim_makespan"], ball.info()["sim_busy"]
     sm_, sb_ = np.array(singles_ms), np.array(singles_busy)
-    sim = {"busy_batched": info["sim_busy"], "busy_one_at_a_time_work_weighted": float((sm_ * sb_).sum() / sm_.sum()),
+    sim = {"busy_batched": batched_busy, "busy_one_at_a_time_work_weighted": float((sm_ * sb_).sum() / sm_.sum()),
            "busy_one_at_a_time_min": float(sb_.min()),
            "predicted_speedup_vs_unbatched": float(sm_.sum() / batched_ms),
-           "note": "host-side list-scheduling simulation of the planner (task durations from their wavefront "
-                   "steps): one problem alone already keeps the SMs this busy, so a shared launch can recover "
-                   "at most the difference"}
+           "note": "host-side list-scheduling simulation of the planner (task durations from the cells of "
+                   "their rows): one problem alone already keeps the SMs this busy, so a shared launch can "
+                   "recover at most the difference"}
     s = torch.cuda.Stream(device=dev)
     sh = s.cuda_stream
 

@@ -469,11 +469,23 @@ int msb_batch_sync(msb_batch* b, void* stream);
  * problem's last task (device clock).  After msb_batch_sync. */
 int msb_batch_problem_ms(const msb_batch* b, double* ms, int n);
 int msb_batch_info(const msb_batch* b, msb_batch_info_t* info);
-/* Host-only planning of the same batch for nsm SMs (no device, pointers may
- * be NULL) for host-side checks; bit k of tile24_mask, k = 0, 1, 2 for nm 4,
- * 8, 16, selects the 2 x 4 tile for that group. */
+/* Host-only planning for nsm SMs (no device, pointers may be NULL), for
+ * host-side checks and the simulated times of the info.
+ * msb_batch_plan_rows: the plan msb_batch_create makes on a device of nsm SMs,
+ * rows per pipeline and cells per row by the rule (rows 0) or rows (8, 4 or 2)
+ * rows of 4 cells for every problem, as autotune may choose.
+ * msb_batch_plan: the same planner over the staged kernel's tiles, one group
+ * pair a task: 4 x 2, or 2 x 4 where bit k of tile24_mask (k = 0, 1, 2 for nm
+ * 4, 8, 16) says so.  No launch runs this cut. */
+int msb_batch_plan_rows(msb_batch** out, const msb_problem* problems, int nproblem, int nsm,
+                        size_t scratch_bytes, int rows);
 int msb_batch_plan(msb_batch** out, const msb_problem* problems, int nproblem, int nsm,
                    size_t scratch_bytes, int tile24_mask);
+/* How each entry is cut: rows per pipeline (0: a staged tile), cells per row,
+ * angle tiles of the kernel body, and the class (the tasks of a class are one
+ * contiguous range of the table, in class order).  Arrays may be NULL;
+ * returns the entry count. */
+int msb_batch_shapes(const msb_batch* b, int* rows, int* cells, int* angle_tiles, int* cls, int max_entries);
 /* A batch sweeps every problem in entries of 32 angles, as a Sweeper sweeps
  * them in passes: entry e is problem problem[e]'s angles [angle0[e],
  * angle0[e] + 32); later entries of a problem add to vo after the entry

@@ -150,6 +150,8 @@ def lib() -> ctypes.CDLL:
                                        ctypes.c_size_t, ctypes.c_int]
         L.msb_batch_plan.argtypes = [P(ctypes.c_void_p), P(ProblemDesc), ctypes.c_int, ctypes.c_int,
                                      ctypes.c_size_t, ctypes.c_int]
+        L.msb_batch_plan_rows.argtypes = L.msb_batch_plan.argtypes
+        L.msb_batch_shapes.argtypes = [ctypes.c_void_p] + [P(ctypes.c_int)] * 4 + [ctypes.c_int]
         L.msb_batch_destroy.argtypes = [ctypes.c_void_p]
         L.msb_batch_destroy.restype = None
         L.msb_batch_sweep.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p]
@@ -596,15 +598,19 @@ class Batch:
 
     `problems`: dicts with the sizes (ncell_x, ncell_y, ncell_z, ne, na, nm)
     and device pointers (vi, vo, a_from_m, m_from_a).  With `plan_nsm` set,
-    only the host-side plan is built (no GPU; pointers may be absent)."""
+    only the host-side plan is built (no GPU; pointers may be absent): the
+    device's plan for that many SMs with `plan_rows` 0 (shapes by the rule) or
+    8, 4, 2 (rows per pipeline), the staged kernel's tiles without."""
 
     def __init__(self, problems: list, precision: int = 0, scratch_bytes: int = 0, autotune: bool = False,
-                 plan_nsm: int = 0, tile24_mask: int = 0):
+                 plan_nsm: int = 0, tile24_mask: int = 0, plan_rows: int = -1):
         L = lib()
         self.n = len(problems)
         self._h = ctypes.c_void_p()
         d = _descs(problems)
-        if plan_nsm:
+        if plan_nsm and plan_rows >= 0:
+            rc = L.msb_batch_plan_rows(ctypes.byref(self._h), d, self.n, plan_nsm, scratch_bytes, plan_rows)
+        elif plan_nsm:
             rc = L.msb_batch_plan(ctypes.byref(self._h), d, self.n, plan_nsm, scratch_bytes, tile24_mask)
         else:
             rc = L.msb_batch_create(ctypes.byref(self._h), d, self.n, precision, scratch_bytes, int(autotune))
@@ -646,6 +652,17 @@ class Batch:
         IP = ctypes.POINTER(ctypes.c_int)
         L.msb_batch_entries(self._h, prob.ctypes.data_as(IP), a0.ctypes.data_as(IP), n)
         return prob, a0
+
+    def shapes(self):
+        """(rows per pipeline, cells per row, angle tiles, class) of every entry."""
+        L = lib()
+        n = L.msb_batch_entries(self._h, None, None, 0)
+        if n < 0:
+            raise SweepError(n, last_error())
+        out = np.zeros((4, n), dtype=np.int32)
+        IP = ctypes.POINTER(ctypes.c_int)
+        L.msb_batch_shapes(self._h, *(r.ctypes.data_as(IP) for r in out), n)
+        return tuple(out)
 
     def tasks(self):
         """(table: ntask x 16 ints with global dependency ids, entry of each task)."""

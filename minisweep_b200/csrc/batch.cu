@@ -138,7 +138,7 @@ struct ProbPlan {
   int user = 0, pass = 0, npass = 1, a0 = 0, nac = 0;
   int prev = -1, next = -1;  // entries of the neighbouring passes
   int nch = 0, ngp = 0, kind = 0, cls = 0, tx = 4, ty = 2;
-  int rw = 0;  // rows per pipeline of the row kernel; 0: planned for the given tile only (no device)
+  int rw = 0;  // rows per pipeline of the row kernel; 0: planned in the staged kernel's tiles
   int nt = 4;  // angle tiles of the class: those of the problem's first pass
   Schedule sched;
   size_t face_bytes[3] = {0, 0, 0};
@@ -582,9 +582,9 @@ int simulate_and_order(BatchImpl& B) {
   return MSB_OK;
 }
 
-// How a batch is cut: on a device for the row kernel (`rows` gives a moment
-// count's rows per pipeline; 0 or absent: the rule's choice per problem),
-// else (host-only plans) in tiles of 4 x 2, or 2 x 4 where `tile24` says so.
+// How a batch is cut: for the row kernel as on a device (`rows` gives a moment
+// count's rows per pipeline; 0 or absent: the rule's choice per problem), else
+// (msb_batch_plan) in tiles of 4 x 2, or 2 x 4 where `tile24` says so.
 struct Shape {
   bool device = false;
   std::map<int, int> rows;
@@ -894,49 +894,41 @@ struct msb_batch {
 };
 
 static int batch_build(msb_batch** out, const msb_problem* problems, int nproblem, int precision,
-                       size_t scratch_bytes, int autotune_flag, int nsm_plan) {
+                       size_t scratch_bytes, int autotune_flag) {
   if (!out || !problems || nproblem <= 0) return msb::set_error(MSB_ERR_ARG, "batch: no problems");
   *out = nullptr;
   if (precision != 0) return msb::set_error(MSB_ERR_UNSUPPORTED, "batch: precision %d (batches sweep in FP64)", precision);
-  const bool device = nsm_plan <= 0;
   int rc;
   for (int i = 0; i < nproblem; ++i)
-    if ((rc = msb::check_problem(problems[i], i, device))) return rc;
+    if ((rc = msb::check_problem(problems[i], i, true))) return rc;
   std::unique_ptr<msb_batch> b(new (std::nothrow) msb_batch());
   if (!b) return msb::set_error(MSB_ERR_ARG, "out of host memory");
   BatchImpl& B = b->impl;
-  if (device) {
-    if ((rc = msb::setup_kernel(&B.nsm))) return rc;
-  } else {
-    B.nsm = nsm_plan;
-  }
+  if ((rc = msb::setup_kernel(&B.nsm))) return rc;
   // arena: the given size, or all the face scratch the problems would need
   // at once, capped at 80 % of the free device memory
-  size_t cap = ~(size_t)0;
-  if (device) {
-    size_t fr = 0, tot = 0;
-    if ((rc = msb::cuda_check(cudaMemGetInfo(&fr, &tot), "cudaMemGetInfo"))) return rc;
-    cap = (size_t)(fr * 0.8);
-  }
+  size_t fr = 0, tot = 0;
+  if ((rc = msb::cuda_check(cudaMemGetInfo(&fr, &tot), "cudaMemGetInfo"))) return rc;
+  const size_t cap = (size_t)(fr * 0.8);
   msb::Shape shape;
   shape.device = true;
-  if (autotune_flag && device) {
+  if (autotune_flag) {
     if ((rc = msb::autotune(problems, nproblem, B.nsm, scratch_bytes ? scratch_bytes : cap, &shape.rows, &b->tune_ms)))
       return rc;
   }
   if ((rc = msb::plan_batch(B, problems, nproblem, shape, scratch_bytes, cap))) return rc;
-  if (device && (rc = msb::upload_batch(B))) return rc;
+  if ((rc = msb::upload_batch(B))) return rc;
   *out = b.release();
   return MSB_OK;
 }
 
 extern "C" int msb_batch_create(msb_batch** out, const msb_problem* problems, int nproblem, int precision,
                                 size_t scratch_bytes, int autotune) {
-  return batch_build(out, problems, nproblem, precision, scratch_bytes, autotune, 0);
+  return batch_build(out, problems, nproblem, precision, scratch_bytes, autotune);
 }
 
-extern "C" int msb_batch_plan(msb_batch** out, const msb_problem* problems, int nproblem, int nsm,
-                              size_t scratch_bytes, int tile24_mask) {
+static int batch_plan(msb_batch** out, const msb_problem* problems, int nproblem, int nsm, size_t scratch_bytes,
+                      const msb::Shape& shape) {
   if (nsm <= 0) return msb::set_error(MSB_ERR_ARG, "batch plan: nsm must be positive");
   if (!out || !problems || nproblem <= 0) return msb::set_error(MSB_ERR_ARG, "batch: no problems");
   *out = nullptr;
@@ -945,15 +937,29 @@ extern "C" int msb_batch_plan(msb_batch** out, const msb_problem* problems, int 
     if ((rc = msb::check_problem(problems[i], i, false))) return rc;
   std::unique_ptr<msb_batch> b(new (std::nothrow) msb_batch());
   if (!b) return msb::set_error(MSB_ERR_ARG, "out of host memory");
-  BatchImpl& B = b->impl;
-  B.nsm = nsm;
+  b->impl.nsm = nsm;
+  if ((rc = msb::plan_batch(b->impl, problems, nproblem, shape, scratch_bytes, ~(size_t)0))) return rc;
+  *out = b.release();
+  return MSB_OK;
+}
+
+extern "C" int msb_batch_plan_rows(msb_batch** out, const msb_problem* problems, int nproblem, int nsm,
+                                   size_t scratch_bytes, int rows) {
+  if (rows != 0 && rows != 8 && rows != 4 && rows != 2)
+    return msb::set_error(MSB_ERR_ARG, "batch plan: rows must be 0, 2, 4 or 8");
+  msb::Shape shape;
+  shape.device = true;
+  for (int nm : {4, 8, 16}) shape.rows[nm] = rows;
+  return batch_plan(out, problems, nproblem, nsm, scratch_bytes, shape);
+}
+
+extern "C" int msb_batch_plan(msb_batch** out, const msb_problem* problems, int nproblem, int nsm,
+                              size_t scratch_bytes, int tile24_mask) {
   // bit (nm index) of the mask selects the 2 x 4 tile
   msb::Shape shape;
   const int nms[3] = {4, 8, 16};
   for (int k = 0; k < 3; ++k) shape.tile24[nms[k]] = ((tile24_mask >> k) & 1) != 0;
-  if ((rc = msb::plan_batch(B, problems, nproblem, shape, scratch_bytes, ~(size_t)0))) return rc;
-  *out = b.release();
-  return MSB_OK;
+  return batch_plan(out, problems, nproblem, nsm, scratch_bytes, shape);
 }
 
 extern "C" void msb_batch_destroy(msb_batch* b) { delete b; }
@@ -1067,6 +1073,20 @@ extern "C" int msb_batch_entries(const msb_batch* b, int* problem, int* angle0, 
   for (int p = 0; p < ne && p < max_entries; ++p) {
     if (problem) problem[p] = B.probs[p].user;
     if (angle0) angle0[p] = B.probs[p].a0;
+  }
+  return ne;
+}
+
+extern "C" int msb_batch_shapes(const msb_batch* b, int* rows, int* cells, int* angle_tiles, int* cls,
+                                int max_entries) {
+  if (!b) return msb::set_error(MSB_ERR_ARG, "batch: invalid argument");
+  const BatchImpl& B = b->impl;
+  const int ne = (int)B.probs.size();
+  for (int p = 0; p < ne && p < max_entries; ++p) {
+    if (rows) rows[p] = B.probs[p].rw;
+    if (cells) cells[p] = B.probs[p].tx;
+    if (angle_tiles) angle_tiles[p] = B.probs[p].nt;
+    if (cls) cls[p] = B.probs[p].cls;
   }
   return ne;
 }

@@ -201,3 +201,117 @@ def test_plan_workload_subset_with_reuse():
         assert np.all(dep[has] < np.arange(len(rec))[has])
         assert np.all(prob[dep[has]] == prob[has])
     assert b.info()["npred"] > 0
+
+
+# ---- the plan a device runs (the row kernel's cut)
+
+ROWS = SMALL + [
+    dict(ncell_x=8, ncell_y=3, ncell_z=40, ne=7, na=45, nm=8),    # a thin region, two passes
+    dict(ncell_x=20, ncell_y=9, ncell_z=6, ne=25, na=24, nm=16),  # 13 group pairs
+    dict(ncell_x=13, ncell_y=17, ncell_z=5, ne=10, na=16, nm=8),  # 5 group pairs, a row more than two pipelines
+]
+
+
+def check_rows_plan(b, problems, rows):
+    """The table's protocol, as check_plan, for the row kernel: blocks of group
+    pairs, one class per (moments, angle tiles), a shape per problem."""
+    rec, prob = b.tasks()
+    n = len(rec)
+    eprob, ea0 = b.entries()
+    rw, tx, nt, cls = b.shapes()
+    off, nb, _, _ = b.scratch()
+    for p, pr in enumerate(problems):
+        mine = np.nonzero(eprob == p)[0]
+        assert list(ea0[mine]) == list(range(0, pr["na"], 32))
+        assert np.all(np.diff(mine) == 1)
+    for d in DEPS:
+        has = rec[:, d] >= 0
+        assert np.all(rec[has, d] < np.arange(n)[has])
+        assert np.all(prob[rec[has, d]] == prob[has])
+    # one contiguous range per class, in class order; a class is one body
+    assert np.all(np.diff(cls[prob]) >= 0)
+    body = {}
+    for e in range(len(eprob)):
+        pr = problems[eprob[e]]
+        assert nt[e] == min(4, -(-pr["na"] // 8))
+        assert body.setdefault(cls[e], (pr["nm"], nt[e])) == (pr["nm"], nt[e])
+        assert rw[e] in (2, 4, 8) and tx[e] in (1, 2, 4) and (not rows or (rw[e], tx[e]) == (rows, 4))
+        # the records: the schedule of blocks of 8 / rw group pairs
+        ngp = (pr["ne"] + 1) // 2
+        nblk = -(-ngp // (8 // rw[e]))
+        own = msb.schedule(pr["ncell_x"], pr["ncell_y"], pr["ncell_z"], 2 * nblk, tx[e], rw[e], 1)
+        mine = np.nonzero(prob == e)[0]
+        key = lambda a: np.lexsort(a.T[::-1])
+        got, want = rec[mine][:, :TK_FLAGS + 1], own[:, :TK_FLAGS + 1]
+        assert np.array_equal(got[key(got)], want[key(want)])
+        pos = {tuple(r[:TK_Z1 + 1]): mine[i] for i, r in enumerate(rec[mine])}
+        ident = {tuple(r[:TK_Z1 + 1]): r for r in own}
+        for r in rec[mine]:
+            o = ident[tuple(r[:TK_Z1 + 1])]
+            for d in DEPS:
+                assert r[d] == (pos[tuple(own[o[d]][:TK_Z1 + 1])] if o[d] >= 0 else -1)
+        # face planes of every octant, group pair and position, nt x 8 angles of 8 columns
+        entry = 8 * ngp * nt[e] * 64 * 8
+        sizes = [entry * pr["ncell_y"] * pr["ncell_x"], entry * pr["ncell_z"] * pr["ncell_x"],
+                 entry * pr["ncell_z"] * pr["ncell_y"]]
+        assert sum(sizes) <= nb[e] <= sum(sizes) + 3 * 256 and nb[e] % 256 == 0 and off[e] % 256 == 0
+    assert len(set(body.values())) == len(body) <= 12
+    return rec, prob
+
+
+@pytest.mark.parametrize("rows", [0, 8, 4, 2])
+@pytest.mark.parametrize("nsm", [1, 8, 148])
+def test_rows_plan(rows, nsm):
+    with msb.Batch(ROWS, plan_nsm=nsm, plan_rows=rows) as b:
+        check_rows_plan(b, ROWS, rows)
+
+
+@pytest.mark.parametrize("rows", [0, 4])
+@pytest.mark.parametrize("nsm", [3, 148])
+def test_rows_plan_reuse_is_ordered(rows, nsm):
+    with msb.Batch(ROWS, plan_nsm=nsm, plan_rows=rows) as probe:
+        size = int(probe.scratch()[1].max())
+    with msb.Batch(ROWS, plan_nsm=nsm, plan_rows=rows, scratch_bytes=size) as b:
+        rec, prob = check_rows_plan(b, ROWS, rows)
+        off, nb, po, pred = b.scratch()
+        first = np.array([np.nonzero(prob == e)[0][0] for e in range(len(off))])
+        last = np.array([np.nonzero(prob == e)[0][-1] for e in range(len(off))])
+        waits = [set(pred[po[e]:po[e + 1]]) for e in range(len(off))]
+        order = np.argsort(first)
+        for e in order:  # transitively
+            for q in list(waits[e]):
+                assert last[q] < first[e]
+                waits[e] |= waits[q]
+        overlaps = 0
+        for e in order:
+            for q in order:
+                if first[e] < first[q] and off[e] < off[q] + nb[q] and off[q] < off[e] + nb[e]:
+                    overlaps += 1
+                    assert last[e] < first[q] and e in waits[q]
+        assert overlaps > 0
+
+
+@pytest.mark.parametrize("nx,ny,nz,ne,shape", [
+    (64, 64, 64, 64, (8, 4)),  # whole pipelines
+    (48, 20, 48, 32, (4, 4)),  # regions of 10 rows: 8 + 2
+    (40, 6, 40, 64, (4, 4)),   # of 3 rows, more tasks than SMs in any shape
+    (20, 4, 6, 64, (2, 4)),    # of 2 rows
+    (8, 2, 64, 2, (8, 1)),     # one row: an SM for each tile of one cell
+    (8, 2, 64, 16, (8, 2)),    # ... of two cells
+    (8, 2, 64, 32, (4, 2)),    # ... two group pairs a CTA
+    (8, 2, 64, 64, (2, 2)),    # ... four
+    (8, 2, 64, 128, (2, 4)),   # ... and whole rows
+    (16, 2, 64, 2, (8, 4)),    # two tiles of whole rows overlap as they are
+    (8, 2, 6, 2, (8, 4)),      # too short to gain
+])
+def test_row_shapes(nx, ny, nz, ne, shape):
+    with msb.Batch([dict(ncell_x=nx, ncell_y=ny, ncell_z=nz, ne=ne, na=32, nm=16)], plan_nsm=148, plan_rows=0) as b:
+        rw, tx, _, _ = b.shapes()
+    assert (rw[0], tx[0]) == shape
+
+
+def test_rows_plan_rejects():
+    with pytest.raises(msb.SweepError):
+        msb.Batch(ROWS, plan_nsm=8, plan_rows=3)
+    with pytest.raises(msb.SweepError):
+        msb.Batch(ROWS, plan_nsm=8, plan_rows=0, scratch_bytes=1024)
