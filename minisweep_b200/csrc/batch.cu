@@ -156,18 +156,18 @@ struct ClassInfo {
 };
 
 // relative cost of one wavefront step of a task (one cell column per warp)
-double step_cost(int nm, int nch) { return (0.3 + 0.7 * nm / 16.0) * nch; }
+double step_cost(int nm) { return 0.3 + 0.7 * nm / 16.0; }
 
 // Duration of a task and the delay until its first plane is through every
 // row.  Row kernel: in cells of a warp, the rows one cell apart.
 void task_times(const ProbPlan& P, const int* r, double* dur, double* plane_delay) {
   const int w = r[TK_X1] - r[TK_X0], h = r[TK_Y1] - r[TK_Y0], nz = r[TK_Z1] - r[TK_Z0];
   if (P.rw) {
-    const double c = step_cost(P.d.nm, 1) * (0.2 + 0.2 * P.nt) / 4.0;
+    const double c = step_cost(P.d.nm) * (0.2 + 0.2 * P.nt) / 4.0;
     *dur = c * (nz * w + h - 1);
     *plane_delay = c * (w + h - 1);
   } else {
-    const double c = step_cost(P.d.nm, P.nch);
+    const double c = step_cost(P.d.nm);
     *dur = c * (nz + w + h - 2);
     *plane_delay = c * (w + h - 1);
   }

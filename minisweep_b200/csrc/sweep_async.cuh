@@ -13,11 +13,11 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
 __device__ __forceinline__ void mbar_init(uint64_t* b, int count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(b)), "r"(count) : "memory");
 }
-__device__ __forceinline__ void mbar_arrive(uint64_t* b) {
-  asm volatile(
-      "{\n .reg .b64 st;\n mbarrier.arrive.release.cta.shared::cta.b64 st, [%0];\n}" ::"r"(smem_u32(b))
-      : "memory");
+// The barrier by its 32-bit shared-memory address (bar_...) or a pointer.
+__device__ __forceinline__ void bar_arrive(uint32_t b) {
+  asm volatile("{\n .reg .b64 st;\n mbarrier.arrive.release.cta.shared::cta.b64 st, [%0];\n}" ::"r"(b) : "memory");
 }
+__device__ __forceinline__ void mbar_arrive(uint64_t* b) { bar_arrive(smem_u32(b)); }
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* b, uint32_t bytes) {
   asm volatile(
       "{\n .reg .b64 st;\n mbarrier.arrive.expect_tx.release.cta.shared::cta.b64 st, [%0], %1;\n}" ::"r"(
@@ -35,9 +35,10 @@ __device__ __forceinline__ bool mbar_test(uint64_t* b, uint32_t parity) {
   return ok != 0;
 }
 // 16-byte asynchronous copy global -> shared (L2 only) and its groups.
-__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+__device__ __forceinline__ void cp_async16_s(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) { cp_async16_s(smem_u32(dst), src); }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 
 // L2 eviction policies (createpolicy) and the copies / stores that carry one.
@@ -78,26 +79,30 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
 }
 
 // Non-blocking test of a phase (test_wait never suspends the warp).
-__device__ __forceinline__ bool mbar_test_wait(uint64_t* b, uint32_t parity) {
+__device__ __forceinline__ bool bar_test(uint32_t b, uint32_t parity) {
   uint32_t ok;
   asm volatile(
       "{\n .reg .pred p;\n mbarrier.test_wait.parity.acquire.cta.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
       : "=r"(ok)
-      : "r"(smem_u32(b)), "r"(parity)
+      : "r"(b), "r"(parity)
       : "memory");
   return ok != 0;
 }
+__device__ __forceinline__ bool mbar_test_wait(uint64_t* b, uint32_t parity) { return bar_test(smem_u32(b), parity); }
 
 // try_wait with a suspend-time hint: the warp sleeps in hardware until the
 // phase completes or about `ns` nanoseconds pass (no busy polling).
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* b, uint32_t parity, uint32_t ns) {
+__device__ __forceinline__ bool bar_try(uint32_t b, uint32_t parity, uint32_t ns) {
   uint32_t ok;
   asm volatile(
       "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cta.shared::cta.b64 p, [%1], %2, %3;\n selp.u32 %0, 1, 0, p;\n}"
       : "=r"(ok)
-      : "r"(smem_u32(b)), "r"(parity), "r"(ns)
+      : "r"(b), "r"(parity), "r"(ns)
       : "memory");
   return ok != 0;
+}
+__device__ __forceinline__ bool mbar_try_wait(uint64_t* b, uint32_t parity, uint32_t ns) {
+  return bar_try(smem_u32(b), parity, ns);
 }
 
 // Bounded wait on an mbarrier phase by a whole warp.  It does not give up

@@ -133,9 +133,6 @@ __device__ __forceinline__ void st_release_cta(int* p, int v) {
   asm volatile("st.release.cta.shared::cta.s32 [%0], %1;" ::"r"(smem_u32(p)), "r"(v) : "memory");
 }
 __device__ __forceinline__ int ld_volatile(const int* p) { return *reinterpret_cast<const volatile int*>(p); }
-__device__ __forceinline__ void cp_async16_s(uint32_t dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-}
 // Predicated forms: the cell loop stays one basic block, so that the
 // tensor-core products can be scheduled among everything else.
 __device__ __forceinline__ void cp_async16_p(uint32_t dst, const void* src, bool on) {
@@ -195,37 +192,14 @@ __device__ __forceinline__ double lds1(uint32_t p) {
 __device__ __forceinline__ void sts2(uint32_t p, double a, double b) {
   asm volatile("st.shared.v2.f64 [%0], {%1,%2};" ::"r"(p), "d"(a), "d"(b) : "memory");
 }
-__device__ __forceinline__ bool bar_test(uint32_t b, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.test_wait.parity.acquire.cta.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-      : "=r"(ok)
-      : "r"(b), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-// as bar_test, the warp asleep in hardware for up to about 2 us
-__device__ __forceinline__ bool bar_try(uint32_t b, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cta.shared::cta.b64 p, [%1], %2, %3;\n selp.u32 %0, 1, 0, p;\n}"
-      : "=r"(ok)
-      : "r"(b), "r"(parity), "r"(2000)
-      : "memory");
-  return ok != 0;
-}
-__device__ __forceinline__ void bar_arrive(uint32_t b) {
-  asm volatile("{\n .reg .b64 st;\n mbarrier.arrive.release.cta.shared::cta.b64 st, [%0];\n}" ::"r"(b) : "memory");
-}
-
-// Bounded wait of a whole warp until the phases of up to three mbarriers
-// (address 0: none) are complete, asleep in hardware meanwhile; false once the
-// CTA quits (all lanes agree).
-static __device__ __noinline__ bool row_wait(uint32_t b0, uint32_t p0, uint32_t b1, uint32_t p1, uint32_t b2,
-                                             uint32_t p2, int* cnt, SyncArgs s) {
+// Bounded wait of a whole warp until the phases of up to two mbarriers
+// (address 0: none) are complete, asleep in hardware meanwhile, up to about 2
+// us at a time; false once the CTA quits (all lanes agree).
+static __device__ __noinline__ bool row_wait(uint32_t b0, uint32_t p0, uint32_t b1, uint32_t p1, int* cnt,
+                                             SyncArgs s) {
   long long t0 = 0;
   for (;;) {
-    const bool ok = (!b0 || bar_try(b0, p0)) && (!b1 || bar_try(b1, p1)) && (!b2 || bar_try(b2, p2));
+    const bool ok = (!b0 || bar_try(b0, p0, 2000)) && (!b1 || bar_try(b1, p1, 2000));
     if (__all_sync(0xffffffffu, ok)) return true;
     bool give_up = ld_volatile(cnt + RC_QUIT) != 0;
     if (!give_up) {
@@ -289,18 +263,18 @@ __device__ __forceinline__ void row_tasker(const PP& P, int cls, double* smem) {
     return true;
   };
 
-  int plane0[2] = {0, 0};  // first plane of the task being posted, of the one before
+  int plane0 = 0;  // first plane of the task posted last
   int plane_next = 0;
   int preds_done_for = -1;
   for (int k = 0;; ++k) {
     // A task is taken when row 0 enters the last planes of the one before:
     // early enough to wait for its dependencies and lay out its matrices,
     // late enough that a reserved task does not sit behind a whole other one.
-    bool ok = k == 0 || row_wait_count(cnt + RC_PLANES, max(plane_next - 4, plane0[0]), cnt, P.sy, 250);
+    bool ok = k == 0 || row_wait_count(cnt + RC_PLANES, max(plane_next - 4, plane0), cnt, P.sy, 250);
     // the record and the matrix buffer were last used by tasks k - 4 (by the
     // rows, the publisher and the fetcher) and k - 2
     ok = ok && row_wait_count(cnt + RC_PUBLISHED, k - C::NREC + 1, cnt, P.sy, 64) &&
-         row_wait_count(cnt + RC_FETCHED, k - C::NREC + 1, cnt, P.sy, 64) && rows_past(plane0[0]);
+         row_wait_count(cnt + RC_FETCHED, k - C::NREC + 1, cnt, P.sy, 64) && rows_past(plane0);
     int t = -1;
     if (ok && lane == 0 && ld_relaxed(&sync[SY_ABORT]) == 0) {
       if constexpr (BATCH) {
@@ -369,21 +343,19 @@ __device__ __forceinline__ void row_tasker(const PP& P, int cls, double* smem) {
       if (lane == 0) st_release_cta(cnt + RC_QUIT, 1);
       return;
     }
-    plane0[1] = plane0[0];
-    plane0[0] = plane_next;
+    plane0 = plane_next;
     plane_next += r[TK_Z1] - r[TK_Z0];
     if (lane == 0) {
       rec->oct = oct; rec->gp = r[TK_GP];
       rec->x0 = r[TK_X0]; rec->x1 = r[TK_X1]; rec->y0 = r[TK_Y0]; rec->y1 = r[TK_Y1];
       rec->z0 = r[TK_Z0]; rec->z1 = r[TK_Z1];
       rec->flags = r[TK_FLAGS]; rec->depx = depx; rec->depy = depy;
-      rec->task = t; rec->stop = 0; rec->plane0 = plane0[0]; rec->prob = prob;
+      rec->task = t; rec->stop = 0; rec->plane0 = plane0; rec->prob = prob;
       rec->rw = Q.rw;
       rec->q = Q;
     }
     __syncwarp();
     if (lane == 0) st_release_cta(cnt + RC_POSTED, k + 1);
-    (void)plane0[1];
   }
 }
 
@@ -800,7 +772,7 @@ __device__ __forceinline__ void row_compute(const PP& P, double* smem) {
       double fx[NT][2];
       if (x_in) {
         xmask = 3;
-        if (!__all_sync(0xffffffffu, bar_test(xfull, x_ph)) && !row_wait(xfull, x_ph, 0, 0, 0, 0, cnt, P.sy)) {
+        if (!__all_sync(0xffffffffu, bar_test(xfull, x_ph)) && !row_wait(xfull, x_ph, 0, 0, cnt, P.sy)) {
           cp_async_wait<0>();
           return;
         }
@@ -818,7 +790,7 @@ __device__ __forceinline__ void row_compute(const PP& P, double* smem) {
         // ---- wait for the entering y face and for room for the leaving one
         const uint32_t yb = yfull + 8 * yi, eb = yempty + 8 * (DY + yo);
         if (!__all_sync(0xffffffffu, bar_test2(yb, yi_ph, y_feed, eb, yo_ph, y_pass)) &&
-            !row_wait(y_feed ? yb : 0, yi_ph, y_pass ? eb : 0, yo_ph, 0, 0, cnt, P.sy)) {
+            !row_wait(y_feed ? yb : 0, yi_ph, y_pass ? eb : 0, yo_ph, cnt, P.sy)) {
           cp_async_wait<0>();
           return;
         }

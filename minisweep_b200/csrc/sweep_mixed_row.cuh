@@ -387,7 +387,7 @@ __device__ __forceinline__ void mix_row_compute(const PP& P, double* smem) {
       float fx[S][4];
       if (x_in) {
         xmask = 3;
-        if (!__all_sync(0xffffffffu, bar_test(xfull, x_ph)) && !row_wait(xfull, x_ph, 0, 0, 0, 0, cnt, P.sy)) {
+        if (!__all_sync(0xffffffffu, bar_test(xfull, x_ph)) && !row_wait(xfull, x_ph, 0, 0, cnt, P.sy)) {
           cp_async_wait<0>();
           return;
         }
@@ -417,7 +417,7 @@ __device__ __forceinline__ void mix_row_compute(const PP& P, double* smem) {
           // ---- wait for the entering y face and for room for the leaving one
           const uint32_t yb = yfull + 8 * yi, eb = yempty + 8 * (DY + yo);
           if (!__all_sync(0xffffffffu, bar_test2(yb, yi_ph, y_feed, eb, yo_ph, y_pass)) &&
-              !row_wait(y_feed ? yb : 0, yi_ph, y_pass ? eb : 0, yo_ph, 0, 0, cnt, P.sy)) {
+              !row_wait(y_feed ? yb : 0, yi_ph, y_pass ? eb : 0, yo_ph, cnt, P.sy)) {
             cp_async_wait<0>();
             return;
           }

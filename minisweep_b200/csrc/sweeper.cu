@@ -440,10 +440,12 @@ static int impl_create(SweeperImpl& S, const Dimensions& dims, int precision, in
   // face entries and angle passes of every plan the sweeper may run
   size_t entry_bytes = S.var.entry_bytes;
   int pass_min = S.var.pass, pass_max = S.var.pass;
+  bool copies = !S.var.rw;  // a plan whose passes need their matrices copied (the row kernels read them in place)
   for (const auto& a : S.alts) {
     entry_bytes = std::max(entry_bytes, a.var.entry_bytes);
     pass_min = std::min(pass_min, a.var.pass);
     pass_max = std::max(pass_max, a.var.pass);
+    copies = copies || !a.var.rw;
   }
   S.sync_ints = SY_PROGRESS + (size_t)ntask;
   if ((rc = cuda_check(cudaMalloc(&S.d_sync, S.sync_ints * sizeof(int)), "cudaMalloc sync"))) return rc;
@@ -465,7 +467,7 @@ static int impl_create(SweeperImpl& S, const Dimensions& dims, int precision, in
   const size_t nmat = (size_t)dims.nm * dims.na * NOCTANT;
   if ((rc = cuda_check(cudaMalloc(&S.d_afm, nmat * sizeof(double)), "cudaMalloc a_from_m"))) return rc;
   if ((rc = cuda_check(cudaMalloc(&S.d_mfa, nmat * sizeof(double)), "cudaMalloc m_from_a"))) return rc;
-  if (dims.na > pass_min) {
+  if (copies && dims.na > pass_min) {
     const size_t npass_mat = (size_t)dims.nm * pass_max * NOCTANT;
     if ((rc = cuda_check(cudaMalloc(&S.d_afm_c, npass_mat * sizeof(double)), "cudaMalloc a_from_m pass"))) return rc;
     if ((rc = cuda_check(cudaMalloc(&S.d_mfa_c, npass_mat * sizeof(double)), "cudaMalloc m_from_a pass"))) return rc;

@@ -142,3 +142,18 @@ def test_sliced_run_reports_timeout_and_recovers():
         pb.set_timeout_ns(0)
         got = host_iterations(pb, vi, 2)
     assert np.array_equal(got, ref)
+
+
+@pytest.mark.parametrize("nx,ny,nz,rows", [(40, 6, 70, 4), (48, 4, 80, 2)])
+@pytest.mark.parametrize("prec", [0, 1])
+def test_sliced_tasks_of_several_group_pairs(nx, ny, nz, rows, prec):
+    """Pipelines of 4 and 2 rows: a task covers 2 or 4 group pairs, which stay
+    in one slice; 33 group pairs leave the last task (and slice) one of them."""
+    extra = f"--precision {prec}" if prec else ""
+    with msb.Problem(flags(nx, ny, nz, 65, 24, extra), nm=16) as pb:
+        assert pb.tile()["ty"] == rows
+        vi = random_state(pb, 11)
+        ref = device_iterations(pb, vi, 2)
+        got = host_iterations(pb, vi, 2)
+        assert pb.iterations_slices() == 4
+    assert np.array_equal(got, ref)
