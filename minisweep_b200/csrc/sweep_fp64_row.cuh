@@ -565,17 +565,21 @@ __device__ __forceinline__ void row_publisher(const PP& P, double* smem) {
 }
 
 // Which of a task's warps a compute warp of the CTA is.  A scheduler holds the
-// warps w and w + 4; numbered so, the rows in use of a task with fewer rows
-// than its pipelines have (rows 0, or 0 and 1, of each pipeline) are on
-// different schedulers as far as there are four.
-__device__ __forceinline__ int row_warp(int w) { return (0x54672310 >> (4 * w)) & 7; }
+// warps w and w + 4.  Pipelines of 4 or 2 rows may have rows to spare: numbered
+// so, the rows in use (rows 0, or 0 and 1, of each pipeline) are on different
+// schedulers as far as there are four.  With 8 rows the rows that share a
+// scheduler are four cells apart as they come.
+__device__ __forceinline__ int row_warp(int w, bool packed) { return packed ? (0x54672310 >> (4 * w)) & 7 : w; }
 
 // One compute warp: row `warp % rw` of pipeline `warp / rw` of each task.
 template <int NM_, int NT, bool BATCH, class PP>
 __device__ __forceinline__ void row_compute(const PP& P, double* smem) {
   using C = RowCfg<NM_, NT>;
   constexpr int E = C::E, VSZ = C::VSZ, W = C::W, D = C::D, DY = C::DY, R = C::R, KS = C::KS, MT = C::MT;
-  const int lane = threadIdx.x & 31, warp = row_warp(__shfl_sync(0xffffffffu, threadIdx.x >> 5, 0));
+  const int lane = threadIdx.x & 31, phys = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
+  int warp;
+  if constexpr (BATCH) warp = row_warp(phys, true);  // one numbering for tasks of any height
+  else warp = row_warp(phys, P.pr.rw < 8);
   const int q = lane >> 2, r = lane & 3;
   int* const cnt = reinterpret_cast<int*>(smem + C::SM_CNT);
   // shared-memory addresses of this warp's barriers, rings and face slots
