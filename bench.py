@@ -129,7 +129,7 @@ def measured_peaks() -> dict:
         return {"hbm_gbs": 6650.0, "bf16_tflops": 1590.0, "source": "fallback (earlier measurement on this pool)"}
 
 
-def profile_traffic(kernel: str = "sweep_fp64_row_kernel") -> float | None:
+def profile_traffic(kernel: str) -> float | None:
     """DRAM bytes per 64^3 sweep of a kernel from its committed ncu summary."""
     try:
         with open(os.path.join(ROOT, "profiles", kernel + ".md")) as f:
@@ -343,10 +343,10 @@ def measure_mixed(args, pb64, flags, va, vb, stream, dev, world, ms_fp64=None) -
 
 def measure_dense(args, dev, world: int, local_rank: int) -> dict | None:
     """The angle/group-heavy case: 32x32x96 cells, ne 128, na 128, NM 16,
-    nblock_z 12, built-in Quantities.  One FP64 sweep (kernel, tile shape,
-    task window and angle passes autotuned by the untimed first sweep) against one sweep of each
-    mixed precision (four 32-angle passes), each timed after one untimed
-    sweep; under torchrun each rank sweeps its own 128-group slice.  The FP64
+    nblock_z 12, built-in Quantities.  One FP64 sweep (kernel, shape, task
+    window and angle passes autotuned by the untimed first sweep) against one
+    sweep of each mixed precision (four 32-angle passes), each timed after one
+    untimed sweep; under torchrun each rank sweeps its own 128-group slice.  The FP64
     sweep of the built-in problem returns its input exactly, so the mixed
     errors are measured against the initial state."""
     if args.no_dense:
@@ -670,9 +670,10 @@ def run_ours(args, rank: int, world: int, local_rank: int) -> int:
     IE_BASE = NE * rank
     flags = (f"--ncell_x {NX} --ncell_y {NY} --ncell_z {NZ} --ne {NE} --na {NA} --nblock_z {NBLOCK_Z} "
              f"--niterations {NITER} --ie_base {IE_BASE}")
-    # --autotune 1: the first (warm-up) sweep times every candidate plan
-    # (both FP64 kernels x both tile shapes x task windows) and keeps the
-    # fastest for every later sweep; --fp64-flags fixes the plan instead
+    # --autotune 1: the first (warm-up) sweep times every candidate plan (the
+    # row kernel's shapes; the staged and the chained kernel x both tile shapes
+    # x task windows) and keeps the fastest for every later sweep; --fp64-flags
+    # fixes the plan instead
     pb = msb.Problem(flags + " " + (args.fp64_flags or "--autotune 1"), nm=NM)
     n = pb.nstate
     va = torch.empty(n, dtype=torch.float64, device=dev)
@@ -740,12 +741,19 @@ def run_ours(args, rank: int, world: int, local_rank: int) -> int:
         tf = flops_per_sweep() / (ms_sweep * 1e-3) / 1e12
         hbm_bytes = 16.0 * NX * NY * NZ * NE * NM * NU  # read vi once, write vo once
         peaks = measured_peaks()
-        traffic = profile_traffic()
+        # of the plan's kernel (the chained one has no scaled capture; the row
+        # kernel's is of pipelines of 8 rows)
+        prof, of = {0: ("sweep_fp64_kernel", "ne 32 sweep scaled x16"),
+                    2: ("sweep_fp64_row_kernel", "ne 16 sweep scaled x32")}.get(tile["fp64_kernel"], (None, None))
+        if tile["fp64_kernel"] == 2 and tile["ty"] != 8:
+            prof = None
+        traffic = profile_traffic(prof) if prof else None
         roofline = {"bound": "tensor", "achieved": tf, "peak": peak_dmma, "unit": "TFLOP/s",
                     "frac": tf / peak_dmma if peak_dmma else None,
                     "traffic": traffic,
-                    "traffic_source": "constant read from profiles/sweep_fp64_row_kernel.md: ncu DRAM bytes of one "
-                                      "32^3 x ne 16 sweep scaled x32 to this workload; not measured in this run",
+                    "traffic_source": f"constant read from profiles/{prof}.md: ncu DRAM bytes of one 32^3 x {of} "
+                                      "to this workload; not measured in this run" if prof else
+                                      "no scaled ncu capture of the plan in use",
                     "peak_source": "FP64 mma.sync peak measured live by msb_measure_fp64_peak (MEASURED_PEAKS.json "
                                    "has no FP64 figure); FMA-pipe FP64 peak %.2f TF/s" % peak_dfma,
                     "algorithmic": "reference flop model (runner.c:162-166) %.4g flop per sweep / mean sweep "

@@ -232,8 +232,7 @@ __device__ __forceinline__ void mix_row_compute(const PP& P, double* smem) {
   using C = MixRowCfg<NM_, FMT, NT>;
   using HF = Half16<FMT>;
   constexpr int E = C::E, W = C::W, D = C::D, DY = C::DY, R = C::R, H = C::H, MT = C::MT, S = C::S, PAIR = C::PAIR;
-  const int lane = threadIdx.x & 31;
-  const int warp = row_warp(__shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), P.pr.rw < 8);
+  const int lane = threadIdx.x & 31, warp = row_warp(P.pr.rw < 8);
   const int q = lane >> 2, r = lane & 3;
   int* const cnt = reinterpret_cast<int*>(smem + C::SM_CNT);
   const uint32_t sb = smem_u32(smem);
