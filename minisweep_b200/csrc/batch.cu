@@ -85,6 +85,9 @@ __device__ __forceinline__ void row_batch_switch(const Fp64Batch& P, int c, doub
   asm volatile("barrier.sync 0;" ::: "memory");
 }
 
+// One numbering of the warps for tasks of any height.
+constexpr bool kSpare = true;
+
 // The classes of a launch come in increasing kind order (the host sorts them
 // so), and the kernel visits the kinds in that order, one straight-line
 // region per kind.
@@ -107,7 +110,7 @@ __global__ void __launch_bounds__(384, 1) sweep_fp64_row_batch_kernel(const Fp64
 #define MSB_K(NM, NT)                                              \
   if (c < P.nclass && P.cls_kind[c] == batch_kind(NM, NT)) {       \
     row_batch_switch(P, c, smem);                                  \
-    row_compute<NM, NT, true>(P, smem);                                  \
+    row_compute<NM, NT, true, kSpare>(P, smem);                          \
     ++c;                                                           \
   }
     MSB_ROW_BATCH_KINDS(MSB_K)
@@ -643,7 +646,7 @@ int plan_batch(BatchImpl& B, const msb_problem* probs, int n, const Shape& shape
         rs = {ir->second, 4};
       else  // the problem's share of the SMs; other problems fill the CTAs: no least number of tasks
         rs = pick_rows(probs[i].ncell_x, probs[i].ncell_y, probs[i].ncell_z, (probs[i].ne + 1) / 2,
-                       (int)(B.nsm * updates(i) / all), 0);
+                       std::max(1, (int)(B.nsm * updates(i) / all)), 0);
     }
     for (int c = 0; c < npass; ++c) {
       ProbPlan e;

@@ -85,6 +85,10 @@ struct RowShape {
   int rw, tx;
 };
 
+// At most half the rows of a pipeline of 4 or 2 are in use: the kernels then
+// number their warps so that those are on different schedulers (row_warp).
+inline bool rows_spare(int ny, int rw) { return rw < 8 && 2 * ((ny + 1) / 2) <= rw; }
+
 // The shape for a problem that has `slots` SMs to itself.  Regions of more
 // than 4 rows get fewer than 8 rows a pipeline only if a cut into 8 would
 // give min_tasks tasks to a phase.

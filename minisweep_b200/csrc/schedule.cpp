@@ -266,22 +266,25 @@ int pick_gp_block(int nx, int ny, int ngp, int tx, int ty, int window) {
 namespace {
 
 // Regions of at most 4 rows.  A task is then one chain of cells after
-// another on few warps, and how long the chain is matters as soon as a
-// phase's tasks find an SM each: group pairs share a CTA (fewer rows a
-// pipeline) only when they have to, and a row is cut in tiles of 2 or 1
-// cells, which follow each other plane by plane, where there are SMs for the
-// tiles.  A tile's plane takes 0.75 us a cell, but 1.2 at least; a tile more
-// in a row costs about 6 cells.  More pipelines in a CTA: a few per cent with
-// 2, 10 to 30 with 4 (their rows share the schedulers then).  A row is cut
-// only where one tile of 4 cells is all of it: with two tiles or more the
-// octants' phases overlap instead.
+// another on few warps, and a phase takes the longer of that chain and of its
+// tasks' share of an SM.  In cells of a warp alone (0.75 us at 16 moments and
+// 32 angles): a task's start and end 14, a tile more in a row 5 and its own
+// first plane; a plane of one cell counts 1.5 (publishing it takes that long);
+// a cell 1.03 with several pipelines in a CTA, 1.3 with more than 4 warps in
+// use.  Group pairs thus share a CTA only once a phase has more tasks than
+// SMs, and a row is cut in tiles of 2 or 1 cells, which follow each other
+// plane by plane, where there are SMs for the tiles; but only where one tile
+// of 4 cells is all of it: with more tiles the octants' phases overlap
+// instead.
 // Measured, us per sweep, nm 16, na 32 (staged kernel; 8 rows x 4 cells; the
 // shape chosen):
 //   8 x 2 x 64, ne 2    496   801  475 (8 x 1)   ne 64   824  1375  667 (2 x 2)
 //   8 x 4 x 64, ne 16   616   837  572 (8 x 2)   ne 128 1919  2794 1129 (2 x 4)
-//   16 x 2 x 64, ne 64 1583  2744 1048 (2 x 4)
+//   16 x 2 x 64, ne 64 1583  2744 1048 (2 x 4)   40 x 4 x 10, ne 16: 442 (8 x 4),
+//   429 (4 x 4, chosen), 488 (2 x 4)
 // The staged kernel stays ahead at 9 to 18 group pairs, nm 16 and 5 to 8 cells
-// along x, by 9 % at most (8 x 2 x 96, ne 32: 735 us, 801 with the 2 x 4 chosen).
+// along x, by 7 % at most (8 x 2 x 96, ne 32: 735 us, 788 with the 4 x 2 chosen).
+// False: regions of 3 or 4 rows and too many tasks, left to the rule below.
 bool pick_thin(int nx, int ny, int nz, int ngp, int slots, RowShape* out) {
   const int hx = (nx + 1) / 2, h0 = (ny + 1) / 2, hz = (nz + 1) / 2;
   double best = 0.0;
@@ -289,17 +292,19 @@ bool pick_thin(int nx, int ny, int nz, int ngp, int slots, RowShape* out) {
     if (tx < 4 && (hx > 4 || tx >= hx)) continue;
     for (int rw : {8, 4, 2}) {
       if (rw < 8 && (h0 > 2 || tx == 1)) break;
-      const long long tasks = (long long)(ceil_div(hx, tx) + ceil_div(nx / 2, tx)) *
-                              (ceil_div(h0, rw) + ceil_div(ny / 2, rw)) * (nz > 1 ? 2 : 1) * ceil_div(ngp, 8 / rw);
-      if (tasks > slots) continue;
-      const double chain = hz * std::max<double>(std::min(tx, hx), 1.5) + 6.0 * (ceil_div(hx, tx) - 1);
-      // a pipeline of 3 or 4 rows: only for a clear gain
-      const double v = chain * (rw == 8 ? 1.0 : rw == 4 ? 1.05 : 1.2) * (tx < 4 && h0 > 2 ? 1.2 : 1.0);
-      if (best == 0.0 || v < best) {
+      const double tasks = (double)(ceil_div(hx, tx) + ceil_div(nx / 2, tx)) *
+                           (ceil_div(h0, rw) + ceil_div(ny / 2, rw)) * (nz > 1 ? 2 : 1) * ceil_div(ngp, 8 / rw);
+      if (tasks > slots && (tx < 4 || h0 > 2)) continue;
+      const int pipes = std::min(8 / rw, ngp), w = std::min(tx, hx);
+      const double cell = pipes * std::min(h0, rw) > 4 ? 1.3 : pipes > 1 ? 1.03 : 1.0;
+      const double task = 14.0 + cell * hz * std::max<double>(w, 1.5);
+      const double chain = task + (ceil_div(hx, tx) - 1) * (5.0 + cell * w);
+      // rows of 3 or 4: cut only for a clear gain
+      const double v = std::max(chain, task * tasks / slots) * (tx < 4 && h0 > 2 ? 1.15 : 1.0);
+      if (best == 0.0 || v < 0.999 * best) {
         best = v;
         *out = {rw, tx};
       }
-      break;
     }
   }
   return best > 0.0;

@@ -565,25 +565,25 @@ __device__ __forceinline__ void row_publisher(const PP& P, double* smem) {
 }
 
 // Which of a task's warps a compute warp of the CTA is.  A scheduler holds the
-// warps w and w + 4.  Pipelines of 4 or 2 rows may have rows to spare: numbered
-// so, the rows in use (rows 0, or 0 and 1, of each pipeline) are on different
-// schedulers as far as there are four.  With 8 rows the rows that share a
-// scheduler are four cells apart as they come.  The shuffle comes last: it
-// tells the compiler that the number is the warp's (64^3 x 64: 57.9 ms, 59.7
-// with arithmetic behind it).
-__device__ __forceinline__ int row_warp(bool packed) {
+// warps w and w + 4.  Where a pipeline of 4 or 2 rows uses half of them at
+// most (SPARE), the rows in use (rows 0, or 0 and 1, of each pipeline) are put
+// on different schedulers: 8 x 2 x 96, ne 32, two pipelines of one row, 788 us
+// instead of 1014.  With more rows in use the plain order is the better one
+// (47 x 6 x 9, ne 77, 3 rows of 4, mixed: 1.04 ms, 1.13 so).  A constant of the
+// kernel, and the shuffle last, which tells the compiler that the number is
+// the warp's: 64^3 x 64 took 59.7 ms instead of 57.6 with arithmetic behind it.
+template <bool SPARE>
+__device__ __forceinline__ int row_warp() {
   const int w = threadIdx.x >> 5;
-  return __shfl_sync(0xffffffffu, packed ? (0x54672310 >> (4 * w)) & 7 : w, 0);
+  return __shfl_sync(0xffffffffu, SPARE ? (0x54672310 >> (4 * w)) & 7 : w, 0);
 }
 
 // One compute warp: row `warp % rw` of pipeline `warp / rw` of each task.
-template <int NM_, int NT, bool BATCH, class PP>
+template <int NM_, int NT, bool BATCH, bool SPARE, class PP>
 __device__ __forceinline__ void row_compute(const PP& P, double* smem) {
   using C = RowCfg<NM_, NT>;
   constexpr int E = C::E, VSZ = C::VSZ, W = C::W, D = C::D, DY = C::DY, R = C::R, KS = C::KS, MT = C::MT;
-  bool packed = true;  // a batch: one numbering for tasks of any height
-  if constexpr (!BATCH) packed = P.pr.rw < 8;
-  const int lane = threadIdx.x & 31, warp = row_warp(packed);
+  const int lane = threadIdx.x & 31, warp = row_warp<SPARE>();
   const int q = lane >> 2, r = lane & 3;
   int* const cnt = reinterpret_cast<int*>(smem + C::SM_CNT);
   // shared-memory addresses of this warp's barriers, rings and face slots
@@ -939,7 +939,7 @@ __device__ __forceinline__ void row_producers(const PP& P, int cls, double* smem
   else if (warp == C::R + 2) row_publisher<C, BATCH>(P, smem);
 }
 
-template <int NM_, int NT>
+template <int NM_, int NT, bool SPARE>
 __global__ void __launch_bounds__(RowCfg<NM_, NT>::NTH, 1) sweep_fp64_row_kernel(const Fp64Params P) {
   using C = RowCfg<NM_, NT>;
   extern __shared__ __align__(128) double smem[];
@@ -951,7 +951,7 @@ __global__ void __launch_bounds__(RowCfg<NM_, NT>::NTH, 1) sweep_fp64_row_kernel
     row_producers<C, false>(P, 0, smem);
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(208));
-    row_compute<NM_, NT, false>(P, smem);
+    row_compute<NM_, NT, false, SPARE>(P, smem);
   }
 }
 

@@ -227,12 +227,12 @@ struct MixRowCfg {
 // One compute warp, as row_compute of the FP64 kernel; Q.vi is the converted
 // vi (kViBlock bytes per (cell, group pair)), Q.vo the octants' FP32 partials
 // (one state after another).
-template <int NM_, int FMT, int NT, class PP>
+template <int NM_, int FMT, int NT, bool SPARE, class PP>
 __device__ __forceinline__ void mix_row_compute(const PP& P, double* smem) {
   using C = MixRowCfg<NM_, FMT, NT>;
   using HF = Half16<FMT>;
   constexpr int E = C::E, W = C::W, D = C::D, DY = C::DY, R = C::R, H = C::H, MT = C::MT, S = C::S, PAIR = C::PAIR;
-  const int lane = threadIdx.x & 31, warp = row_warp(P.pr.rw < 8);
+  const int lane = threadIdx.x & 31, warp = row_warp<SPARE>();
   const int q = lane >> 2, r = lane & 3;
   int* const cnt = reinterpret_cast<int*>(smem + C::SM_CNT);
   const uint32_t sb = smem_u32(smem);
@@ -575,7 +575,7 @@ __device__ __forceinline__ void mix_row_compute(const PP& P, double* smem) {
   }
 }
 
-template <int NM_, int FMT, int NT>
+template <int NM_, int FMT, int NT, bool SPARE>
 __global__ void __launch_bounds__(384, 1) sweep_mixed_row_kernel(const Fp64Params P) {
   using C = MixRowCfg<NM_, FMT, NT>;
   extern __shared__ __align__(128) double smem[];
@@ -586,7 +586,7 @@ __global__ void __launch_bounds__(384, 1) sweep_mixed_row_kernel(const Fp64Param
     row_producers<C, false>(P, 0, smem);
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(208));
-    mix_row_compute<NM_, FMT, NT>(P, smem);
+    mix_row_compute<NM_, FMT, NT, SPARE>(P, smem);
   }
 }
 

@@ -91,12 +91,12 @@ Variant make_chain_variant() {
 // The row kernel (sweep_fp64_row.cuh): rw rows of tx <= 4 cells per pipeline,
 // 8 / rw pipelines (group pairs) per CTA.
 template <int NM_>
-Variant make_row_variant(RowShape shape, int na) {
+Variant make_row_variant(RowShape shape, bool spare, int na) {
   Variant v;
-  v.row_fn[0] = sweep_fp64_row_kernel<NM_, 1>;
-  v.row_fn[1] = sweep_fp64_row_kernel<NM_, 2>;
-  v.row_fn[2] = sweep_fp64_row_kernel<NM_, 3>;
-  v.row_fn[3] = sweep_fp64_row_kernel<NM_, 4>;
+  v.row_fn[0] = spare ? sweep_fp64_row_kernel<NM_, 1, true> : sweep_fp64_row_kernel<NM_, 1, false>;
+  v.row_fn[1] = spare ? sweep_fp64_row_kernel<NM_, 2, true> : sweep_fp64_row_kernel<NM_, 2, false>;
+  v.row_fn[2] = spare ? sweep_fp64_row_kernel<NM_, 3, true> : sweep_fp64_row_kernel<NM_, 3, false>;
+  v.row_fn[3] = spare ? sweep_fp64_row_kernel<NM_, 4, true> : sweep_fp64_row_kernel<NM_, 4, false>;
   v.row_smem[0] = RowCfg<NM_, 1>::smem_bytes();
   v.row_smem[1] = RowCfg<NM_, 2>::smem_bytes();
   v.row_smem[2] = RowCfg<NM_, 3>::smem_bytes();
@@ -116,11 +116,12 @@ Variant make_row_variant(RowShape shape, int na) {
   return v;
 }
 
-Variant pick_row(int nm, int na, RowShape shape) {
-  switch (nm) {
-    case 4: return make_row_variant<4>(shape, na);
-    case 8: return make_row_variant<8>(shape, na);
-    case 16: return make_row_variant<16>(shape, na);
+Variant pick_row(const Dimensions& d, RowShape shape) {
+  const bool spare = rows_spare(d.ncell_y, shape.rw);
+  switch (d.nm) {
+    case 4: return make_row_variant<4>(shape, spare, d.na);
+    case 8: return make_row_variant<8>(shape, spare, d.na);
+    case 16: return make_row_variant<16>(shape, spare, d.na);
     default: return Variant();
   }
 }
@@ -140,12 +141,12 @@ Variant pick_nch(int nch, int tile) {
 
 // The mixed-precision row kernel (bodies for passes of 16 and 32 angles).
 template <int NM_, int FMT>
-Variant make_mixed(RowShape shape, int na) {
+Variant make_mixed(RowShape shape, bool spare, int na) {
   static_assert(MixRowCfg<NM_, FMT, 4>::smem_bytes() <= 227 * 1024, "shared memory budget");
   Variant v;
   v.mix = true;
-  v.row_fn[1] = sweep_mixed_row_kernel<NM_, FMT, 2>;
-  v.row_fn[3] = sweep_mixed_row_kernel<NM_, FMT, 4>;
+  v.row_fn[1] = spare ? sweep_mixed_row_kernel<NM_, FMT, 2, true> : sweep_mixed_row_kernel<NM_, FMT, 2, false>;
+  v.row_fn[3] = spare ? sweep_mixed_row_kernel<NM_, FMT, 4, true> : sweep_mixed_row_kernel<NM_, FMT, 4, false>;
   v.row_smem[1] = MixRowCfg<NM_, FMT, 2>::smem_bytes();
   v.row_smem[3] = MixRowCfg<NM_, FMT, 4>::smem_bytes();
   v.conv = convert_vi16<NM_, FMT>;
@@ -164,11 +165,11 @@ Variant make_mixed(RowShape shape, int na) {
 }
 
 template <int FMT>
-Variant pick_mixed(int nm, RowShape shape, int na) {
+Variant pick_mixed(int nm, RowShape shape, bool spare, int na) {
   switch (nm) {
-    case 4: return make_mixed<4, FMT>(shape, na);
-    case 8: return make_mixed<8, FMT>(shape, na);
-    case 16: return make_mixed<16, FMT>(shape, na);
+    case 4: return make_mixed<4, FMT>(shape, spare, na);
+    case 8: return make_mixed<8, FMT>(shape, spare, na);
+    case 16: return make_mixed<16, FMT>(shape, spare, na);
     default: return Variant();
   }
 }
@@ -186,11 +187,11 @@ Variant pick_chain(int tile) {
 // 32-angle chunks per pass (matrices read from shared memory; slower per
 // angle).  na <= 128; the mixed kernels sweep 32 angles per pass.
 Variant pick_variant(int nm, int na, int precision, int tile = 0, int kernel = 0, int angle_pass = 0,
-                     RowShape shape = {8, 4}) {
+                     RowShape shape = {8, 4}, bool spare = false) {
   if (na > 128) return Variant();
   if (precision == 1 || precision == 2) {
     if (tile != 0) return Variant();
-    return precision == 1 ? pick_mixed<MIX_F16>(nm, shape, na) : pick_mixed<MIX_BF16>(nm, shape, na);
+    return precision == 1 ? pick_mixed<MIX_F16>(nm, shape, spare, na) : pick_mixed<MIX_BF16>(nm, shape, spare, na);
   }
   if (precision != 0) return Variant();
   if (kernel == 1) {
@@ -383,9 +384,10 @@ static int impl_create(SweeperImpl& S, const Dimensions& dims, int precision, in
   S.nsm = nsm;
   // no flag asks for a shape or a kernel: the row kernel
   const RowShape shape = pick_rows(dims.ncell_x, dims.ncell_y, dims.ncell_z, S.ngp, nsm, 4 * nsm);
-  if (S.var.mix) S.var = pick_variant(dims.nm, dims.na, precision, 0, 0, 0, shape);
+  if (S.var.mix)
+    S.var = pick_variant(dims.nm, dims.na, precision, 0, 0, 0, shape, rows_spare(dims.ncell_y, shape.rw));
   if (precision == 0 && kernel == 0 && tile == 0 && angle_pass == 0 && !autotune)
-    S.var = pick_row(dims.nm, dims.na, shape);
+    S.var = pick_row(dims, shape);
   if ((rc = setup_plan(S, S.var, S.window, S.sched, S.gp_block, S.d_tasks, S.grid))) return rc;
   long long ntask = S.sched.ntask();
   if (autotune) {
@@ -405,7 +407,7 @@ static int impl_create(SweeperImpl& S, const Dimensions& dims, int precision, in
     if (shape.tx != 4) rows.push_back(shape);
     for (const RowShape& r : rows) {
       AltPlan a;
-      a.var = pick_row(dims.nm, dims.na, r);
+      a.var = pick_row(dims, r);
       a.window = S.window;
       a.l2_hints = S.l2_hints;
       if ((rc = setup_plan(S, a.var, a.window, a.sched, a.gp_block, a.d_tasks, a.grid))) {
