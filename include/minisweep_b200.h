@@ -342,7 +342,9 @@ int Sweeper_sweep_iterations(Sweeper* sweeper, double* v_out_h, const double* v_
  * the results are the same.  No reference counterpart. */
 int msb_iterations_slices(const Sweeper* sweeper);
 /* Device-side FP64 checksums of two device state arrays (same sums as
- * get_state_norms). */
+ * get_state_norms).  With an Env the workspace is kept for the next call until
+ * an Env is finalised (at most 32 MiB a device); env NULL: the default stream,
+ * nothing kept. */
 int msb_state_norms_device(const double* vi_d, const double* vo_d, size_t n,
                            double* normsq, double* normsqdiff, Env* env);
 /* Device-side built-in initial state (same values as initialize_state). */
@@ -354,7 +356,8 @@ int msb_initialize_state_device(double* v_d, Dimensions dims, Env* env);
 int msb_initialize_state_slice_device(double* v_d, Dimensions dims, int ie_base, Env* env);
 /* Kernel statistics of the last sweep: number of tasks, kernel launches. */
 int Sweeper_last_stats(const Sweeper* sweeper, long long* ntask, int* nlaunch);
-/* Tile shape (cell columns per CTA) the sweeper uses and, with --autotune 1,
+/* Tile shape (cell columns per CTA; row kernel: cells per row and rows per
+ * pipeline) the sweeper uses and, with --autotune 1,
  * the first sweep's times (ms) of the chosen plan and of the fastest plan
  * with the other tile shape (0 before that sweep, or without autotuning).
  * No reference counterpart: the reference's --ncell_{x,y}_per_subblock size
@@ -366,8 +369,9 @@ int Sweeper_tile(const Sweeper* sweeper, int* tx, int* ty, float* ms_chosen, flo
  * (--angle_pass; na above it is swept in passes).  With --autotune 1 the
  * first sweep runs every candidate -- the staged and the chained kernel (the
  * staged one with 64- and with 32-angle passes when na > 32) x both tile
- * shapes x task windows 4, 8 and 16, and the row kernel's pipelines -- and
- * keeps the fastest.  No reference counterpart (the
+ * shapes x task windows 4, 8 and 16, the row kernel's pipelines and the
+ * shape of a sweeper without flags -- and keeps the fastest (regions of at
+ * most 4 rows and 4 planes: row kernel 4 x 2 only).  No reference counterpart (the
  * reference's tuning flags, sweeper_kba_c.h:54-233, are set by hand). */
 int Sweeper_plan(const Sweeper* sweeper, int* fp64_kernel, int* task_window, int* l2_hints, int* ncandidates,
                  int* angle_pass);
@@ -426,7 +430,8 @@ int msb_sweep_noalloc(double* vo_d, const double* vi_d, const double* a_from_m_d
  * need at once, capped at 80 % of the free device memory); problems that do
  * not fit at once reuse the bytes of problems that completed earlier in the
  * same launch.  Every problem is swept by the row kernel in pipelines of 8, 4
- * or 2 rows of 4 cells (class_tx x class_ty of the info is the smallest, 4 x 2);
+ * or 2 rows of 4 cells, thin ones of 2 or 1 (class_tx x class_ty of the info is
+ * the smallest of whole rows, 4 x 2);
  * autotune != 0 times these on the median problem of each nm group at
  * creation; those trial sweeps write that problem's vo.  Asynchronous calls run on the
  * given stream (a cudaStream_t, NULL = the legacy default stream); their

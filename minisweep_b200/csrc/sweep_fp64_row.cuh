@@ -10,16 +10,18 @@
 // warps drift apart, and while one waits or solves the other warps keep the
 // FP64 pipe busy.
 //
-// rw = 8, 4 or 2 rows form one pipeline (a tile of 4 x rw cells); a CTA then
-// holds 1, 2 or 4 pipelines, each on a group pair of its own.
+// rw = 8, 4 or 2 rows form one pipeline (a tile of 4 x rw cells; 2 or 1 cells
+// wide where a region is so narrow that one tile would be all of its row); a
+// CTA then holds 1, 2 or 4 pipelines, each on a group pair of its own.
 //
 // What bounds it: per cell, group pair and octant a warp issues 32 FP64
 // tensor-core products (m8n8k4, 16 cycles of the scheduler's FP64 pipe each)
 // and 56 FP64 instructions of the solve (2 cycles each): 624 cycles at 16
 // moments and 32 angles, 1250 for the two warps of a scheduler; and 3 KB of
 // state and 4 KB (1/4 + 1/rw) of faces cross L2.  Measured, 64^3 cells x 64
-// groups, ms per sweep: 57.6 (rw 8; 2040 cycles per two cells, DRAM at 4.9
-// TB/s), 63.0 (rw 2), the staged kernel 120.2.  What got it there from 92:
+// groups, ms per sweep on the built-in inputs: 57.6 (rw 8; 2040 cycles per two
+// cells, DRAM at 4.9 TB/s), 63.0 (rw 2), the staged kernel 120.2; on random
+// inputs 63 to 68 from one card to another.  What got it there from 92:
 // the vi / vo copies issued by the compute warps themselves (one warp feeding
 // all eight by bulk copies was the bound: 92 -> 81), then a cell body without
 // branches, in which the next cell's first product, the solve and the second
@@ -33,7 +35,8 @@
 //             and posts the task to the other warps.
 //   fetcher   brings the faces entering the tile once the upwind tile's
 //             progress covers their plane, one 1-D bulk copy each: lane w the
-//             x faces of compute warp w, lane 8 + p the y faces of pipeline p.
+//             x faces of row w, lane 8 + w the y faces of row w where it is a
+//             pipeline's first.
 //   publisher follows the rows' plane counts and publishes the task's
 //             progress (planes every row has finished) to global memory.
 //
@@ -68,8 +71,9 @@ struct RowCfg {
   // input ring of a warp, in cells: 4 x 2 KB at 16 moments; a cell of 8 or 4
   // moments takes less time and less room
   static constexpr int D = NM_ == 16 ? 4 : NM_ == 8 ? 6 : 8;
-  // y faces between two rows: as many as fit, since the rows do not run
-  // evenly (37 x 29 x 41, ne 23, na 45, nm 8: 6.53 ms with 3, 6.23 so)
+  // y faces between two rows: up to 6, as far as they fit beside the rest,
+  // since the rows do not run evenly (37 x 29 x 41, ne 23, na 45, nm 8: 6.53
+  // ms with 3, 6.23 so)
   static constexpr int DY = NT <= 2 ? 6 : NT == 3 ? 5 : NM_ == 16 ? 3 : NM_ == 8 ? 4 : 5;
   static constexpr int NREC = 4;              // task records
   static constexpr int MAT = (KS + MT * 2) * NT * 32;

@@ -37,9 +37,10 @@
 // What bounds it: instruction issue (55 % of the slots with two warps per
 // scheduler): about 430 warp instructions a cell, 190 of them the FP32 solve
 // with its error terms, 18 products.  Measured, ms per sweep (conversion and
-// partial sum included): 64^3 x 64 groups 66.5 (FP16) / 67.3 (BF16), the
-// CTA-wide form 91.6 / 92.8; 64^3 x 16 16.6 / 23.4.  With 12 rows and 128
-// registers 16.5: the third warp gains what 32 rows in tiles of 12 lose.
+// partial sum included): 64^3 x 64 groups 63.0 (FP16) / 64.0 (BF16), the
+// CTA-wide form 91.6 / 92.8; 64^3 x 16 15.7 / 23.4.  With 12 rows and 128
+// registers no faster (16.5 where this one then took 16.6): the third warp
+// gains what 32 rows in tiles of 12 lose.
 #pragma once
 
 #include <cuda_bf16.h>

@@ -732,8 +732,9 @@ static int impl_sync(SweeperImpl& S, cudaStream_t stream) {
 // with its own task table: the host->device copy of slice k + 1 then runs
 // while slice k is swept, and the device->host copy of slice k while slice
 // k + 1 is.  Every value is the one the unsliced run computes.  Slices are
-// used only where they stay efficient (64^3 cells x na 32, one B200: 115.9 ms
-// per sweep with 64 groups, 58.2 with 32, 29.8 with 16, 16.4 with 8).
+// used only where they stay efficient (64^3 cells x na 32, random state, one
+// B200: 63.0 ms per sweep with 64 groups, 32.4 with 32, 15.9 with 16, 7.8 with
+// 8, each in a cut of its own).
 static int slice_count(const SweeperImpl& S) {
   if (S.kba || !S.var.valid() || (S.autotune && !S.tuned)) return 1;
   const size_t bytes = Dimensions_size_state(S.dims, NU) * sizeof(double);
