@@ -647,9 +647,11 @@ int plan_batch(BatchImpl& B, const msb_problem* probs, int n, const Shape& shape
       auto ir = shape.rows.find(probs[i].nm);
       if (ir != shape.rows.end() && ir->second)
         rs = {ir->second, 4};
-      else  // the problem's share of the SMs; other problems fill the CTAs: no least number of tasks
+      else  // the problem's share of the SMs, of which tasks that wait for others hold some (two
+            // problems, 12 x 1 x 30 and 5 x 6 x 45: 349 us with 3/4, 453 with all, 372 with half);
+            // other problems fill the CTAs: no least number of tasks
         rs = pick_rows(probs[i].ncell_x, probs[i].ncell_y, probs[i].ncell_z, (probs[i].ne + 1) / 2,
-                       std::max(1, (int)(B.nsm * updates(i) / all)), 0);
+                       std::max(1, (int)(B.nsm * (n > 1 ? 0.75 : 1.0) * updates(i) / all)), 0);
     }
     for (int c = 0; c < npass; ++c) {
       ProbPlan e;
